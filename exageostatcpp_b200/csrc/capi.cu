@@ -19,6 +19,7 @@
 #include <cuda.h>
 #include "common.cuh"
 #include "kernels.cuh"
+#include "panel_step.cuh"
 
 namespace egs {
 
@@ -46,6 +47,7 @@ struct egs_problem {
   int* flags = nullptr;  // [0] potrf info, [1] device wait error
   MaternParams* dparams = nullptr;
   double* ktab = nullptr;  // Chebyshev table of K_nu for the current theta (kKtabDoubles)
+  double* pscratch = nullptr;  // solved rows of two panel steps (panel_scratch_doubles)
   // pinned host mirrors
   MaternParams* hparams = nullptr;
   double* hresult = nullptr;
@@ -142,7 +144,6 @@ struct egs_problem {
 namespace {
 
 constexpr int kInnerBlock = 64;
-constexpr int kOuterBlock = 256;
 constexpr int kPrecisionBroken = -1;  // egs_problem_set_precision failed part-way
 
 int round_tile(int dts) {
@@ -304,7 +305,8 @@ void free_mixed(egs_problem* p) {
 void free_problem(egs_problem* p) {
   if (!p) return;
   if (p->stream) cudaStreamSynchronize(p->stream);
-  void* bufs[] = {p->tiles, p->x, p->y, p->z, p->zcpy, p->partial, p->result, p->flags, p->dparams, p->ktab};
+  void* bufs[] = {p->tiles, p->x, p->y, p->z, p->zcpy, p->partial, p->result, p->flags, p->dparams, p->ktab,
+                  p->pscratch};
   for (void* b : bufs) dev_free(b, p->stream);
   free_mixed(p);
   pinned_release(p->hparams);
@@ -318,69 +320,63 @@ void free_problem(egs_problem* p) {
 }
 
 // Panel of step k (tile column k of an nt-tile lower layout): factor diagonal
-// tile (k, k) and solve tiles (k+1 .. nt-1, k) against it, as one right-looking
-// blocked factorisation of the tall tile column.  Two-level blocking: the
-// tile's columns go in outer blocks of kOuterBlock; inside an outer block each
-// 64-column block is factored (64x64 potrf), every row below it -- the rest of
-// the diagonal tile and all tiles below -- is solved in one row-solve launch,
-// and one K = 64 update covers the remaining columns of the same outer block
-// for all those rows; the columns right of the outer block then get one
-// update with K = kOuterBlock.  The K = 64 updates thus touch at most 192
-// columns, which cuts the read-modify-write traffic of the panel's C operand
-// by ~2.5x against single-level 64-blocking.  Every element receives the same
-// operations in the same order as with the diagonal tile factored first.
-// col_base is the global column of the tile (for the LAPACK-style info of a
-// failed pivot).  Returns the launch count in *nl.
-int enqueue_panel(double* tiles, const void* tmap, int ts, int nt, int k, int col_base, int* info, int* err,
-                  cudaStream_t st, long long* nl, int max_ctas = 0) {
-  const long long skk = tile_slot(k, k, nt);
-  const int ntp = nt - k;         // tiles of the column, the diagonal one first
+// tile (k, k) and solve the tiles below it up to tile row row_tiles - 1, as one
+// right-looking blocked factorisation of the tall tile column.  Two-level
+// blocking: the tile's columns go in outer blocks of at most five 64-column
+// blocks; each 64-column step is one launch that also updates the rest of its
+// outer block (panel_step.cuh), and the columns right of the outer block get
+// one update with K = the outer block's width.  col_base is the global column
+// of the tile (for the LAPACK-style info of a failed pivot); z (or null) the
+// segment of tile row k of a vector that becomes L^-1 z along the way.  The
+// last step's solved rows stay in ch's scratch until the next step or
+// launch_panel_flush.  Returns the launch count in *nl.
+int enqueue_panel(double* tiles, const void* tmap, int ts, int nt, int row_tiles, int k, int col_base, int* info,
+                  int* err, double* z, PanelChain& ch, cudaStream_t st, long long* nl, int max_ctas = 0) {
+  double* col = tiles + tile_slot(k, k, nt) * (long long)ts * ts;
   const int drow = k * ts;
-  const int row_end = nt * ts;    // end of the column's global rows
-  for (int KB = 0; KB < ts; KB += kOuterBlock) {
-    const int KE = std::min(ts, KB + kOuterBlock);
-    for (int kb = KB; kb < KE; kb += kInnerBlock) {
-      launch_potrf_diag_block(tiles, ts, skk, kb, col_base, info, st);
-      ++*nl;
-      const int r0 = drow + kb + kInnerBlock;  // first row below the block
-      if (r0 >= row_end) continue;
-      launch_trsm_rows_panel(tiles, ts, skk, ntp, kb + kInnerBlock, 0, kb, skk, st);
-      ++*nl;
-      if (kb + kInnerBlock < KE) {
-        int rc = launch_gemm_rows(tmap, tiles, ts, nt, row_end - r0, KE - kb - kInnerBlock, kInnerBlock, r0, kb, k,
-                                  r0, kb, k, r0, r0, 1, err, st, max_ctas);
-        if (rc != EGS_OK) return rc;
-        ++*nl;
-      }
-    }
+  const int row_end = row_tiles * ts;  // end of the panel's global rows
+  int KB = 0;                          // first column of the current outer block
+  for (int kb = 0; kb < ts; kb += kInnerBlock) {
+    const int nb = panel_outer_blocks(ts, kb) - 1;
+    int rc = launch_panel_step(col, ts, row_end - (drow + kb + kInnerBlock), kb, nb, col_base + kb, info, z, ch, st);
+    if (rc != EGS_OK) return rc;
+    ++*nl;
+    if (nb > 0) continue;
+    const int KE = kb + kInnerBlock;
     if (KE < ts) {
       const int r0 = drow + KE;
-      int rc = launch_gemm_rows(tmap, tiles, ts, nt, row_end - r0, ts - KE, KE - KB, r0, KB, k, r0, KB, k, r0, r0, 1,
-                                err, st, max_ctas);
+      rc = launch_gemm_rows(tmap, tiles, ts, nt, row_end - r0, ts - KE, KE - KB, r0, KB, k, r0, KB, k, r0, r0, 1, err,
+                            st, max_ctas);
       if (rc != EGS_OK) return rc;
       ++*nl;
     }
+    KB = KE;
   }
   return EGS_OK;
 }
 
 // Right-looking tiled Cholesky of the lower tiles (replaces CHAMELEON_dpotrf_Tile).
-// Step k: factor diagonal tile k (64-wide blocked: potrf of the 64x64 block,
-// row solve below it, tensor-core syrk of the rest of the tile), solve the tile
-// column below it (64-wide blocked: row solve + tensor-core update), then the
-// tensor-core trailing update of every tile (i, j), k < j <= i.
-int enqueue_potrf(egs_problem* p, int steps = -1) {
+// Step k: the panel of tile column k (enqueue_panel), then the tensor-core
+// trailing update of every tile (i, j), k < j <= i.  z (or null) is a vector of
+// np entries that becomes L^-1 z with the panels.
+int enqueue_potrf(egs_problem* p, double* z = nullptr, int steps = -1) {
   const int ts = p->ts, nt = p->nt, n = p->n;
   cudaStream_t st = p->stream;
   int* info = p->flags;
   int* err = p->flags + 1;
   const int kend = (steps >= 0 && steps < nt) ? steps : nt;
+  PanelChain ch;
+  ch.scratch = p->pscratch;
   for (int k = 0; k < kend; ++k) {
-    const long long skk = tile_slot(k, k, nt);
     int sp = span_begin(p, EGS_STAGE_PANEL);
     long long nl = 0;
-    int rc = enqueue_panel(p->tiles, p->tmap, ts, nt, k, k * ts, info, err, st, &nl);
+    int rc = enqueue_panel(p->tiles, p->tmap, ts, nt, nt, k, k * ts, info, err,
+                           z ? z + (long long)k * ts : nullptr, ch, st, &nl);
     if (rc != EGS_OK) return rc;
+    if (k == kend - 1) {
+      if ((rc = launch_panel_flush(ch, st)) != EGS_OK) return rc;
+      ++nl;
+    }
     count_launches(p, EGS_STAGE_PANEL, nl);
     // Algorithmic flops of the panel step on the real (unpadded) rows: potrf of the
     // diagonal block plus the triangular solve of the rows below it.
@@ -410,7 +406,7 @@ int enqueue_potrf(egs_problem* p, int steps = -1) {
 // Caller tiles that are not device tiles (dts not a multiple of 64) take the
 // element-level form of the same loop on logical tiles of dts (dst.cu).
 int enqueue_potrf_band(egs_problem* p) {
-  const int ts = p->ts, nt = p->nt, n = p->n, band = p->band;
+  const int ts = p->ts, nt = p->nt, n = p->n, band = std::min(p->band, nt);
   cudaStream_t st = p->stream;
   int* info = p->flags;
   int* err = p->flags + 1;
@@ -422,49 +418,27 @@ int enqueue_potrf_band(egs_problem* p) {
     span_end(p, sp, 0.0);
     return rc;
   }
+  PanelChain ch;
+  ch.scratch = p->pscratch;
   for (int k = 0; k < nt; ++k) {
-    const long long skk = tile_slot(k, k, nt);
     int sp = span_begin(p, EGS_STAGE_PANEL);
-    for (int kb = 0; kb < ts; kb += kInnerBlock) {
-      launch_potrf_diag_block(p->tiles, ts, skk, kb, k * ts, info, st);
-      count_launches(p, EGS_STAGE_PANEL, 1);
-      if (kb + kInnerBlock < ts) {
-        launch_trsm_rows(p->tiles, ts, skk, 1, kb + kInnerBlock, kb, skk, st);
-        const int r0 = k * ts + kb + kInnerBlock;
-        const int m = ts - kb - kInnerBlock;
-        int rc = launch_gemm_rows(p->tmap, p->tiles, ts, nt, m, m, kInnerBlock, r0, kb, k, r0, kb, k, r0, r0, 1,
-                                  err, st);
-        if (rc != EGS_OK) return rc;
-        count_launches(p, EGS_STAGE_PANEL, 2);
-      }
-    }
+    long long nl = 0;
     const int mend = std::min(nt, k + band);  // solved tiles: k < m < mend
-    const int ntl = mend - k - 1;
-    if (ntl > 0) {
-      const long long s0 = tile_slot(k + 1, k, nt);
-      for (int kb = 0; kb < ts; kb += kInnerBlock) {
-        launch_trsm_rows(p->tiles, ts, s0, ntl, 0, kb, skk, st);
-        count_launches(p, EGS_STAGE_PANEL, 1);
-        if (kb + kInnerBlock < ts) {
-          const int ncols = ts - kb - kInnerBlock;
-          const int brow = k * ts + kb + kInnerBlock;
-          int rc = launch_gemm_rows(p->tmap, p->tiles, ts, nt, ntl * ts, ncols, kInnerBlock, (k + 1) * ts, kb, k,
-                                    brow, kb, k, (k + 1) * ts, brow, 0, err, st);
-          if (rc != EGS_OK) return rc;
-          count_launches(p, EGS_STAGE_PANEL, 1);
-        }
-      }
+    int rc = enqueue_panel(p->tiles, p->tmap, ts, nt, mend, k, k * ts, info, err, nullptr, ch, st, &nl);
+    if (rc != EGS_OK) return rc;
+    if (k == nt - 1) {
+      if ((rc = launch_panel_flush(ch, st)) != EGS_OK) return rc;
+      ++nl;
     }
+    count_launches(p, EGS_STAGE_PANEL, nl);
     span_end(p, sp, 0.0);
+    if (mend <= k + 1) continue;
+    // tiles (m, c), k < c < mend, c <= m < min(nt, c + band), in one launch
     sp = span_begin(p, EGS_STAGE_UPDATE);
+    if ((rc = launch_gemm_band(p->tmap, p->tiles, ts, nt, k, band, err, st)) != EGS_OK) return rc;
+    count_launches(p, EGS_STAGE_UPDATE, 1);
     double flops = 0.0;
     for (int c = k + 1; c < mend; ++c) {
-      // tiles (m, c), c <= m < min(nt, c + band): one launch on the global rows of that range
-      const int rows = (std::min(nt, c + band) - c) * ts;
-      int rc = launch_gemm_rows(p->tmap, p->tiles, ts, nt, rows, ts, ts, c * ts, 0, k, c * ts, 0, k, c * ts, c * ts,
-                                1, err, st);
-      if (rc != EGS_OK) return rc;
-      count_launches(p, EGS_STAGE_UPDATE, 1);
       const double rr = (double)std::max(0, std::min(n, std::min(nt, c + band) * ts) - c * ts);
       const double cc = (double)std::max(0, std::min(n, (c + 1) * ts) - c * ts);
       flops += 2.0 * rr * cc * ts - cc * (cc - 1.0) * ts;
@@ -543,13 +517,15 @@ int enqueue_eval(egs_problem* p) {
   if (rc != EGS_OK) return rc;
   count_launches(p, EGS_STAGE_GENERATE, 1 + (lower_tiles(p->nt) + 65534) / 65535);
   span_end(p, sp, 0.0);
-  rc = p->band > 0 ? enqueue_potrf_band(p) : enqueue_potrf(p);
+  // the exact factorisation carries Z := L^-1 Z along; the band approximation
+  // solves fewer rows than the substitution uses, so it solves afterwards
+  rc = p->band > 0 ? enqueue_potrf_band(p) : enqueue_potrf(p, p->z);
   if (rc != EGS_OK) return rc;
   sp = span_begin(p, EGS_STAGE_REDUCE);
   launch_logdet_partials(p->tiles, p->ts, p->nt, p->n, p->partial, st);
   span_end(p, sp, 0.0);
   count_launches(p, EGS_STAGE_REDUCE, 1);
-  enqueue_trsv(p);
+  if (p->band > 0) enqueue_trsv(p);
   sp = span_begin(p, EGS_STAGE_REDUCE);
   launch_finalize(p->partial, p->nt, p->z, p->n, p->result, p->flags, st);
   span_end(p, sp, 0.0);
@@ -635,8 +611,13 @@ static int enqueue_short_panel(egs_problem* p, int k, cudaStream_t s, int max_ct
   int sp = span_begin(p, EGS_STAGE_PANEL, s);
   long long nl = 0;
   launch_gather_panel(p->band_pool, p->W2, ts, b, nb, k, s);
-  if (int rc = enqueue_panel(p->W2, p->tmapW2, ts, nb + 2, 0, k * ts, p->flags, p->flags + 1, s, &nl, max_ctas))
+  PanelChain ch;
+  ch.scratch = p->pscratch;
+  if (int rc = enqueue_panel(p->W2, p->tmapW2, ts, nb + 2, nb + 2, 0, k * ts, p->flags, p->flags + 1, nullptr, ch, s,
+                             &nl, max_ctas))
     return rc;
+  if (int rc = launch_panel_flush(ch, s)) return rc;
+  ++nl;
   launch_scatter_panel(p->W2, p->band_pool, p->inv_pool, p->W, ts, b, nb, k, s);
   count_launches(p, EGS_STAGE_PANEL, nl + 2);
   span_end(p, sp, panel_flops(ts, p->n, k), s);
@@ -733,7 +714,12 @@ int enqueue_eval_mixed(egs_problem* p) {
     ++nl;
     // W holds tile column k and an identity tile as a one-column problem of
     // ntp + 1 tiles; the solve of the identity row gives L_kk^-T
-    if (int rc = enqueue_panel(p->W, p->tmapW, ts, ntp + 1, 0, k * ts, info, err, st, &nl)) return rc;
+    PanelChain ch;
+    ch.scratch = p->pscratch;
+    if (int rc = enqueue_panel(p->W, p->tmapW, ts, ntp + 1, ntp + 1, 0, k * ts, info, err, nullptr, ch, st, &nl))
+      return rc;
+    if (int rc = launch_panel_flush(ch, st)) return rc;
+    ++nl;
     launch_scatter_column(p->W, p->band_pool, p->off_pool, p->inv_pool, ts, nt, b, k, st);
     ++nl;
     if (ntp > 1) {
@@ -766,7 +752,8 @@ int setup_mixed(egs_problem* p, int b) {
   for (void* buf : {(void*)p->tiles, (void*)p->x, (void*)p->y, (void*)p->z, (void*)p->zcpy, (void*)p->partial})
     dev_free(buf, p->stream);
   p->tiles = p->x = p->y = p->z = p->zcpy = p->partial = nullptr;
-  p->bytes = (long long)(sizeof(MaternParams) + kKtabDoubles * sizeof(double) + 2 * sizeof(int) + 4 * sizeof(double));
+  p->bytes = (long long)(sizeof(MaternParams) + (kKtabDoubles + panel_scratch_doubles()) * sizeof(double) +
+                         2 * sizeof(int) + 4 * sizeof(double));
   const int ts = ((std::max(p->dts, 256) + 255) / 256) * 256;
   p->ts = ts;
   p->nt = (p->n + ts - 1) / ts;
@@ -1022,7 +1009,8 @@ static int create_problem(egs_problem** out, int n, int dts, bool with_tiles) {
       (rc = dev_alloc(&p->partial, p->nt, &p->bytes, p->stream)) ||
       (rc = dev_alloc(&p->result, 4, &p->bytes, p->stream)) || (rc = dev_alloc(&p->flags, 2, &p->bytes, p->stream)) ||
       (rc = dev_alloc(&p->dparams, 1, &p->bytes, p->stream)) ||
-      (rc = dev_alloc(&p->ktab, kKtabDoubles, &p->bytes, p->stream))) {
+      (rc = dev_alloc(&p->ktab, kKtabDoubles, &p->bytes, p->stream)) ||
+      (rc = dev_alloc(&p->pscratch, (size_t)panel_scratch_doubles(), &p->bytes, p->stream))) {
     free_problem(p);
     return rc;
   }
@@ -1536,7 +1524,8 @@ constexpr size_t kNoAllocResultOff = kNoAllocPartialOff + kNoAllocMaxTileRows * 
 constexpr size_t kNoAllocFlagsOff = kNoAllocResultOff + 4 * sizeof(double);
 constexpr size_t kNoAllocParamsOff = kNoAllocFlagsOff + 256;
 constexpr size_t kNoAllocKtabOff = kNoAllocParamsOff + 256;
-constexpr size_t kNoAllocScratchBytes = kNoAllocKtabOff + kKtabDoubles * sizeof(double);
+constexpr size_t kNoAllocPanelOff = (kNoAllocKtabOff + kKtabDoubles * sizeof(double) + 255) / 256 * 256;
+constexpr size_t kNoAllocScratchBytes = kNoAllocPanelOff + kScratchDoubles * sizeof(double);
 constexpr int kNoAllocMaxDevices = 64;
 static_assert(sizeof(MaternParams) <= 256, "parameter slot of the static scratch");
 
@@ -1636,6 +1625,7 @@ int egs_mle_eval_noalloc(int n, int dts, const double* x, const double* y, const
   q.flags = flags;
   q.dparams = dparams;
   q.ktab = ktab;
+  q.pscratch = reinterpret_cast<double*>(scratch + kNoAllocPanelOff);
   q.stream = (cudaStream_t)cuda_stream;
   q.own_stream = false;
   if ((rc = gemm_init_tensor_map(q.tmap, q.tiles, q.ts, q.ntiles)) != EGS_OK) return rc;
@@ -1653,9 +1643,8 @@ int egs_mle_eval_noalloc(int n, int dts, const double* x, const double* y, const
     EGS_CUDA_TRY(cudaMemsetAsync(q.z + n, 0, pad, st));
   }
   if ((rc = launch_matern_tiles(q.tiles, q.x, q.y, n, q.ts, q.nt, dparams, ktab, st)) != EGS_OK) return rc;
-  if ((rc = enqueue_potrf(&q)) != EGS_OK) return rc;
+  if ((rc = enqueue_potrf(&q, q.z)) != EGS_OK) return rc;
   launch_logdet_partials(q.tiles, q.ts, q.nt, n, partial, st);
-  enqueue_trsv(&q);
   launch_finalize(partial, q.nt, q.z, n, result, flags, st);
   if ((rc = check_cuda("egs_mle_eval_noalloc")) != EGS_OK) return rc;
   double hres[4];
@@ -1994,7 +1983,7 @@ namespace egs {
 // (augmented matrices).  Returns the LAPACK-style info or an error.
 int enqueue_potrf_steps(egs_problem* p, int steps) {
   EGS_CUDA_TRY(cudaMemsetAsync(p->flags, 0, 2 * sizeof(int), p->stream));
-  int rc = enqueue_potrf(p, steps);
+  int rc = enqueue_potrf(p, nullptr, steps);
   if (rc != EGS_OK) return rc;
   EGS_CUDA_TRY(cudaMemcpyAsync(p->hflags, p->flags, 2 * sizeof(int), cudaMemcpyDeviceToHost, p->stream));
   EGS_CUDA_TRY(cudaStreamSynchronize(p->stream));

@@ -27,6 +27,7 @@
 #include <cudaTypedefs.h>
 #include <cstdint>
 #include "common.cuh"
+#include "dmma.cuh"
 #include "kernels.cuh"
 #include "mbarrier.cuh"
 
@@ -50,29 +51,6 @@ constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 2 * STAGES * 8 + 1024;
 constexpr int GROUP = 8;                              // block-columns per raster group
 }  // namespace gemm
-
-__device__ __forceinline__ double lds_f64(uint32_t addr) {
-  double v;
-  asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(addr));
-  return v;
-}
-__device__ __forceinline__ void lds_v2f64(uint32_t addr, double& a, double& b) {
-  asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(a), "=d"(b) : "r"(addr));
-}
-__device__ __forceinline__ void ldg_v2f64(const double* p, double& a, double& b) {
-  asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(a), "=d"(b) : "l"(p));
-}
-__device__ __forceinline__ void stg_v2f64(double* p, double a, double b) {
-  asm volatile("st.global.v2.f64 [%0], {%1, %2};" ::"l"(p), "d"(a), "d"(b) : "memory");
-}
-__device__ __forceinline__ void dmma_16816(double (&d)[4], const double (&a)[8], const double (&b)[4]) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7,%8,%9,%10,%11}, "
-      "{%12,%13,%14,%15}, {%0,%1,%2,%3};"
-      : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
-      : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(a[4]), "d"(a[5]), "d"(a[6]), "d"(a[7]), "d"(b[0]),
-        "d"(b[1]), "d"(b[2]), "d"(b[3]));
-}
 
 // MMA row g (0..7) of an A fragment -> tile row 2*perm[g] within a 16-row box;
 // row g+8 -> the next row, so (a_2j, a_2j+1) is one 16-byte load.
@@ -116,6 +94,15 @@ __device__ __forceinline__ bool decode_block(long long L, const GemmDesc& d, int
   return false;
 }
 
+// Blocks with nothing to write: above the diagonal, or (band targets of the
+// lower pool, c_mode 2) wholly below the band.
+__device__ __forceinline__ bool block_skipped(const GemmDesc& d, int mb, int nb) {
+  if (d.lower && mb < nb) return true;
+  if (d.c_mode != 2) return false;
+  const int ti = (d.c_row0 + mb * gemm::BM) / d.ts, tj = (d.c_col0 + nb * gemm::BN + gemm::BN - 1) / d.ts;
+  return ti - tj > d.c_band;
+}
+
 // Producer cursor: walks the same (block, k-step) sequence as the consumers,
 // running up to STAGES-1 stages ahead of them.  The TMA (x, z) coordinates of
 // the 2 x 8 boxes of a block depend only on the block, so they are computed
@@ -149,7 +136,7 @@ __device__ __forceinline__ void cursor_seek(Cursor& c, const GemmDesc& single, c
     const GemmDesc& d = *locate_job<kBatched>(c.L, single, J, local);
     int mb, nb;
     decode_block(local, d, mb, nb);
-    if (!(d.lower && mb < nb)) {
+    if (!block_skipped(d, mb, nb)) {
       box_coords(d.a_row0 + mb * gemm::BM, d.a_tcol, d, coords);
       box_coords(d.b_row0 + nb * gemm::BN, d.b_tcol, d, coords + gemm::BM / gemm::BOX_ROWS);
       c.d = &d;
@@ -263,7 +250,7 @@ dgemm_update_kernel(const __grid_constant__ CUtensorMap tmap, double* __restrict
     const GemmDesc& d = *locate_job<kBatched>(L, single, J, local);
     int mb, nb;
     decode_block(local, d, mb, nb);
-    if (d.lower && mb < nb) continue;
+    if (block_skipped(d, mb, nb)) continue;
     const int ksteps = d.K / BK;
     double acc[4][4][4];
 #pragma unroll
@@ -328,7 +315,7 @@ dgemm_update_kernel(const __grid_constant__ CUtensorMap tmap, double* __restrict
           const int gi = d.c_row0 + ml;
           const int ti = gi / ts, lr = gi - ti * ts;
           const bool ok_el = nl < d.N && ml < d.M && ti >= tj && (d.c_mode == 0 || ti - tj <= d.c_band);
-          const long long cslot = d.c_mode == 0 ? d.tile_base + tile_slot(ti, tj, d.nt)
+          const long long cslot = d.c_mode != 1 ? d.tile_base + tile_slot(ti, tj, d.nt)
                                                 : (long long)(d.c_tile_off + tj) * (d.c_band + 1) + (ti - tj);
           ptr[h][mi] = ok_el ? tiles + cslot * (long long)ts * ts + (long long)lc * ts + lr : nullptr;
           if (ok_el) ldg_v2f64(ptr[h][mi], cv[h][mi][0], cv[h][mi][1]);
@@ -447,6 +434,27 @@ int launch_gemm_trailing(const void* tmap, double* tiles, int ts, int nt, int k,
   d.a_col0 = d.b_col0 = 0;
   d.a_tcol = d.b_tcol = k;
   d.lower = 1;
+  return launch_desc(tmap, tiles, d, err, st);
+}
+
+// Update of step k of the band approximation: tiles (m, c), k < c < k + band,
+// c <= m < c + band, in one launch.
+int launch_gemm_band(const void* tmap, double* tiles, int ts, int nt, int k, int band, int* err, cudaStream_t st) {
+  GemmDesc d{};
+  d.ts = ts;
+  d.nt = nt;
+  d.np = nt * ts;
+  const int r0 = (k + 1) * ts;
+  const int cend = nt < k + band ? nt : k + band;               // columns: tiles k+1 .. cend-1
+  const int rend = nt < cend - 1 + band ? nt : cend - 1 + band;  // rows: up to tile rend-1
+  d.M = rend * ts - r0;
+  d.N = cend * ts - r0;
+  d.K = ts;
+  d.a_row0 = d.b_row0 = d.c_row0 = d.c_col0 = r0;
+  d.a_tcol = d.b_tcol = k;
+  d.lower = 1;
+  d.c_mode = 2;
+  d.c_band = band - 1;
   return launch_desc(tmap, tiles, d, err, st);
 }
 

@@ -19,12 +19,28 @@ int launch_matern_block(double* a, int lda, int rows, int cols, const double* x1
 
 // Factorisation building blocks (potrf.cu).  All offsets are element offsets
 // inside a tile; tiles are addressed by lower-tile slot.
-void launch_potrf_diag_block(double* tiles, int ts, long long slot, int off, int col_base, int* info,
-                             cudaStream_t st);
-void launch_trsm_rows(double* tiles, int ts, long long slot0, int ntiles, int row0, int col0,
-                      long long lslot, cudaStream_t st);
-void launch_trsm_rows_panel(double* tiles, int ts, long long slot0, int ntiles, int row0_first, int row0, int col0,
-                            long long lslot, cudaStream_t st);
+// Panel steps of one factorisation (panel_step.cuh): the scratch slots the steps
+// use alternately, and the step whose solved rows are still in its slot.
+struct PanelChain {
+  double* scratch = nullptr;  // panel_scratch_doubles()
+  int parity = 0;             // slot of the next step
+  int chunks = 0;             // 64-row chunks of the last step still in the other slot (0: none)
+  double* col = nullptr;
+  int kb = 0, ts = 0;
+  double* z = nullptr;
+};
+long long panel_scratch_doubles();
+// 64-column blocks from column kb (a multiple of 64) of a ts-wide tile to the end of its outer block.
+int panel_outer_blocks(int ts, int kb);
+// One step: col is tile (k, k) of a contiguous tile column, rows_below the rows
+// under the 64 x 64 block at (kb, kb), nb the further 64-column blocks of its
+// outer block (updated by the step), gcol the global column of the block (for
+// info), z (or null) the segment of tile row k of a vector that becomes L^-1 z.
+// The diagonal block, z's segment and the solved rows inside the outer block
+// reach their place with the next step's launch or launch_panel_flush.
+int launch_panel_step(double* col, int ts, int rows_below, int kb, int nb, int gcol, int* info, double* z,
+                      PanelChain& ch, cudaStream_t st);
+int launch_panel_flush(PanelChain& ch, cudaStream_t st);
 void launch_trsv_diag(const double* tiles, int ts, long long slot, double* zk, cudaStream_t st);
 void launch_gemv_panel(const double* tiles, int ts, int nt, int k, double* z, cudaStream_t st);
 void launch_trsv_t_diag(const double* tiles, int ts, long long slot, double* zk, cudaStream_t st);
@@ -57,7 +73,8 @@ struct GemmDesc {
   long long tile_base;  // slot of this problem's tile (0, 0) in a pool of problems
   // C addressing: c_mode 0 = lower-tile pool (tile_base + tile_slot(ti, tj, nt));
   // c_mode 1 = FP64 band pool of a mixed-precision problem: only tiles with
-  // ti - tj <= c_band are written, at slot (c_tile_off + tj) * (c_band + 1) + (ti - tj).
+  // ti - tj <= c_band are written, at slot (c_tile_off + tj) * (c_band + 1) + (ti - tj);
+  // c_mode 2 = lower-tile pool, only tiles with ti - tj <= c_band.
   int c_mode, c_band, c_tile_off;
 };
 
@@ -76,6 +93,7 @@ int gemm_init_tensor_map(void* tmap_storage, double* tiles, int ts, long long nt
 // The driver's cuTensorMapEncodeTiled (looked up once).
 int tensor_map_encoder(void** fn);
 int launch_gemm_trailing(const void* tmap, double* tiles, int ts, int nt, int k, int* err, cudaStream_t st);
+int launch_gemm_band(const void* tmap, double* tiles, int ts, int nt, int k, int band, int* err, cudaStream_t st);
 int launch_gemm_rows(const void* tmap, double* tiles, int ts, int nt, int M, int N, int K, int a_row0,
                      int a_col0, int a_tcol, int b_row0, int b_col0, int b_tcol, int c_row0, int c_col0,
                      int lower, int* err, cudaStream_t st, int max_ctas = 0);

@@ -1,6 +1,6 @@
-// Panel-level building blocks of the tiled Cholesky path on sm_100a: the 64x64
-// diagonal-block factorisation, the row-parallel triangular solve of a 64-column
-// block, the single right-hand-side forward/backward substitution over tiles,
+// Panel-level building blocks of the tiled Cholesky path on sm_100a: the 64-column
+// panel step (diagonal block, row solve and update in one launch), the single
+// right-hand-side forward/backward substitution over tiles,
 // and the deterministic reductions that turn the factor into the log-likelihood.
 //
 // Reference counterparts:
@@ -17,50 +17,75 @@
 #include "common.cuh"
 #include "kernels.cuh"
 #include "panel_bodies.cuh"
+#include "panel_step.cuh"
 
 namespace egs {
 
-// Cholesky of the 64x64 diagonal block at (off, off) of one tile (potrf64_body).
-__global__ void __launch_bounds__(256)
-potrf_diag_block_kernel(double* __restrict__ tiles, int ts, long long slot, int off, int col_base,
-                        int* __restrict__ info) {
-  potrf64_body<256>(tiles + slot * (long long)ts * ts + (long long)off * ts + off, ts, col_base + off, info);
+// One 64-column step of a panel (panel_step_body), and the flush of the step
+// before it: blocks [0, steps) are the step's row chunks, the others copy the
+// scratch slot of the previous step to its place.
+__global__ void __launch_bounds__(kStepThreads, 512 / kStepThreads)
+panel_step_kernel(double* col, int ts, int nchunk, int kb, int nb, int gcol, int* info, double* z,
+                  double* __restrict__ out, const double* __restrict__ pslot, double* pcol, int pkb, double* pz) {
+  extern __shared__ __align__(16) double step_smem[];
+  const int steps = nchunk > 0 ? nchunk : 1;
+  const int b = blockIdx.x;
+  if (b < steps) {
+    panel_step_body(step_smem, col, ts, nchunk > 0 ? b : -1, kb, nb, gcol, b == 0 ? info : nullptr, z, out);
+  } else {
+    panel_flush_body(pslot, pcol, ts, pkb, b - steps, pz);
+  }
 }
 
-void launch_potrf_diag_block(double* tiles, int ts, long long slot, int off, int col_base, int* info,
-                             cudaStream_t st) {
-  potrf_diag_block_kernel<<<1, 256, 0, st>>>(tiles, ts, slot, off, col_base, info);
+__global__ void __launch_bounds__(kStepThreads)
+panel_flush_kernel(const double* __restrict__ slot, double* __restrict__ col, int ts, int kb, double* __restrict__ z) {
+  panel_flush_body(slot, col, ts, kb, blockIdx.x, z);
 }
 
-// X := A * L^-T for the 64-column block [col0, col0+64) of ntiles consecutive
-// tiles starting at slot0: rows [row0_first, ts) of the first tile and rows
-// [row0, ts) of the others; L is the factored 64x64 diagonal block at (col0,
-// col0) of tile lslot (trsm_rows_body).
-__global__ void __launch_bounds__(128)
-trsm_rows_kernel(double* __restrict__ tiles, int ts, long long slot0, int grid_row0, int row0_first, int row0,
-                 int col0, long long lslot) {
-  const int lo = blockIdx.y == 0 ? row0_first : row0;
-  int row = grid_row0 + blockIdx.x * blockDim.x + threadIdx.x;
-  if (row < lo) row = ts;  // takes part in loading L only
-  trsm_rows_body<128>(tiles + (slot0 + blockIdx.y) * (long long)ts * ts, tiles + lslot * (long long)ts * ts, ts,
-                      row, col0);
+long long panel_scratch_doubles() { return kScratchDoubles; }
+
+int panel_outer_blocks(int ts, int kb) {
+  // a tile's 64-column blocks in as few outer blocks of at most
+  // kStepMaxBlocks as possible, of nearly equal size
+  const int nblk = ts / kStep, parts = (nblk + kStepMaxBlocks - 1) / kStepMaxBlocks;
+  const int q = nblk / parts, rem = nblk % parts, at = kb / kStep;
+  int lo = 0;
+  for (int i = 0; i < parts; ++i) {
+    const int w = q + (i < rem ? 1 : 0);
+    if (at < lo + w) return lo + w - at;
+    lo += w;
+  }
+  return 1;
 }
 
-void launch_trsm_rows(double* tiles, int ts, long long slot0, int ntiles, int row0, int col0,
-                      long long lslot, cudaStream_t st) {
-  launch_trsm_rows_panel(tiles, ts, slot0, ntiles, row0, row0, col0, lslot, st);
+int launch_panel_step(double* col, int ts, int rows_below, int kb, int nb, int gcol, int* info, double* z,
+                      PanelChain& ch, cudaStream_t st) {
+  static std::once_flag done[64];
+  once_per_device(done, []() {
+    cudaFuncSetAttribute(panel_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         panel_step_smem(kStepMaxBlocks - 1));
+  });
+  const int nchunk = rows_below / kStep;
+  double* out = ch.scratch + (long long)ch.parity * kScratchSlot;
+  const double* pslot = ch.scratch + (long long)(ch.parity ^ 1) * kScratchSlot;
+  const int grid = (nchunk > 0 ? nchunk : 1) + ch.chunks;
+  panel_step_kernel<<<grid, kStepThreads, panel_step_smem(nb), st>>>(col, ts, nchunk, kb, nb, gcol, info, z, out,
+                                                                     pslot, ch.col, ch.kb, ch.z);
+  ch.col = col;
+  ch.kb = kb;
+  ch.chunks = 1 + (nb < nchunk ? nb : nchunk);
+  ch.z = z;
+  ch.ts = ts;
+  ch.parity ^= 1;
+  return launch_status("panel_step_kernel");
 }
 
-void launch_trsm_rows_panel(double* tiles, int ts, long long slot0, int ntiles, int row0_first, int row0, int col0,
-                            long long lslot, cudaStream_t st) {
-  if (ntiles <= 0) return;
-  if (ntiles == 1) row0 = row0_first;
-  const int first = row0 < row0_first ? row0 : row0_first;
-  const int rows = ts - first;
-  if (rows <= 0) return;
-  const int threads = 128;
-  trsm_rows_kernel<<<dim3((rows + threads - 1) / threads, ntiles), threads, 0, st>>>(tiles, ts, slot0, first,
-                                                                                    row0_first, row0, col0, lslot);
+int launch_panel_flush(PanelChain& ch, cudaStream_t st) {
+  if (ch.chunks == 0) return EGS_OK;
+  const double* slot = ch.scratch + (long long)(ch.parity ^ 1) * kScratchSlot;
+  panel_flush_kernel<<<ch.chunks, kStepThreads, 0, st>>>(slot, ch.col, ch.ts, ch.kb, ch.z);
+  ch.chunks = 0;
+  return launch_status("panel_flush_kernel");
 }
 
 // Forward substitution on one diagonal tile: z_k := L_kk^-1 z_k (trsv_diag_body).
