@@ -11,10 +11,10 @@
 //    first tile slot, location offset and tile count;
 //  * problems are ordered by tile count (descending), so the problems still
 //    active at factorisation step k are a prefix of that order;
-//  * step k launches the 64x64 diagonal potrf, the row solves and the
-//    tensor-core updates for all active problems at once; the DMMA update runs
-//    a precomputed job table (one job per problem) through the batched mode of
-//    dgemm_update_kernel;
+//  * step k launches the 64-column panel steps (which carry the forward solve)
+//    and the tensor-core updates for all active problems at once; the DMMA
+//    update runs a precomputed job table (one job per problem) through the
+//    batched mode of dgemm_update_kernel;
 //  * the whole evaluation of all problems is captured once as a CUDA graph and
 //    replayed for every new set of theta (one graph launch per optimiser step).
 #include <algorithm>
@@ -28,6 +28,7 @@
 #include "kernels.cuh"
 #include "matern_tile.cuh"
 #include "panel_bodies.cuh"
+#include "panel_step.cuh"
 
 namespace egs {
 
@@ -52,26 +53,32 @@ matern_batch_kernel(double* __restrict__ tiles, const double* __restrict__ x, co
                     (long long)blockIdx.x * kGenPairsPerBlock, prm, stab);
 }
 
-__global__ void __launch_bounds__(256)
-potrf_batch_kernel(double* __restrict__ tiles, int ts, int k, int kb, const long long* __restrict__ tile_base,
-                   const int* __restrict__ ntv, int* __restrict__ info) {
-  const int p = blockIdx.x;
-  const long long slot = tile_base[p] + tile_slot(k, k, ntv[p]);
-  potrf64_body<256>(tiles + slot * (long long)ts * ts + (long long)kb * ts + kb, ts, k * ts + kb, info + p);
-}
-
-// panel = 0: rows [row0, ts) of the diagonal tile; panel = 1: all rows of tiles k+1.. of each problem.
-__global__ void __launch_bounds__(128)
-trsm_batch_kernel(double* __restrict__ tiles, int ts, int k, int row0, int col0, int panel,
-                  const long long* __restrict__ tile_base, const int* __restrict__ ntv) {
-  const int p = blockIdx.z;
-  const int nt = ntv[p];
-  const int ntl = panel ? nt - k - 1 : 1;
-  if ((int)blockIdx.y >= ntl) return;
-  const long long sl = tile_base[p] + tile_slot(k, k, nt);
-  const long long sa = panel ? tile_base[p] + tile_slot(k + 1 + blockIdx.y, k, nt) : sl;
-  trsm_rows_body<128>(tiles + sa * (long long)ts * ts, tiles + sl * (long long)ts * ts, ts,
-                 row0 + blockIdx.x * blockDim.x + threadIdx.x, col0);
+// One 64-column panel step (tile column k, column kb, panel_step_body) of every
+// problem with more than k tile rows, and the flush of the previous step (pk,
+// pkb, pnb) of every problem that had one: blocks x < steps are row chunks, the
+// rest scratch chunks; block y is the problem.
+__global__ void __launch_bounds__(kStepThreads, 512 / kStepThreads)
+panel_step_batch_kernel(double* tiles, int ts, int k, int kb, int nb, int steps, int active, int pk, int pkb, int pnb,
+                        int pactive, int parity, const long long* __restrict__ tile_base, const int* __restrict__ ntv,
+                        int* info, double* z, const long long* __restrict__ loc_base, double* __restrict__ scratch) {
+  extern __shared__ __align__(16) double step_smem[];
+  const int p = blockIdx.y, nt = ntv[p];
+  double* slots = scratch + (long long)p * kScratchDoubles;
+  double* pool = tiles + tile_base[p] * (long long)ts * ts;
+  if ((int)blockIdx.x < steps) {
+    if (p >= active) return;
+    const int nchunk = ((nt - k) * ts - kb) / kStep - 1;
+    if ((int)blockIdx.x >= (nchunk > 0 ? nchunk : 1)) return;
+    panel_step_body(step_smem, pool + tile_slot(k, k, nt) * (long long)ts * ts, ts, nchunk > 0 ? (int)blockIdx.x : -1,
+                    kb, nb, k * ts + kb, blockIdx.x == 0 ? info + p : nullptr, z + loc_base[p] + (long long)k * ts,
+                    slots + parity * kScratchSlot);
+  } else {
+    const int f = blockIdx.x - steps;
+    const int nchunk = p < pactive ? ((nt - pk) * ts - pkb) / kStep - 1 : -1;
+    if (nchunk < 0 || f > min(pnb, nchunk)) return;
+    panel_flush_body(slots + (parity ^ 1) * kScratchSlot, pool + tile_slot(pk, pk, nt) * (long long)ts * ts, ts, pkb,
+                     f, z + loc_base[p] + (long long)pk * ts);
+  }
 }
 
 __global__ void __launch_bounds__(256)
@@ -84,25 +91,6 @@ logdet_batch_kernel(const double* __restrict__ tiles, int ts, const long long* _
   const double s =
       logdet_tile_body(tiles + (tile_base[p] + tile_slot(k, k, ntv[p])) * (long long)ts * ts, ts, rows);
   if (threadIdx.x == 0) partial[partial_base[p] + k] = s;
-}
-
-__global__ void __launch_bounds__(1024)
-trsv_batch_kernel(const double* __restrict__ tiles, int ts, int k, const long long* __restrict__ tile_base,
-                  const int* __restrict__ ntv, double* __restrict__ z, const long long* __restrict__ loc_base) {
-  const int p = blockIdx.x;
-  trsv_diag_body(tiles + (tile_base[p] + tile_slot(k, k, ntv[p])) * (long long)ts * ts, ts,
-                 z + loc_base[p] + (long long)k * ts);
-}
-
-__global__ void __launch_bounds__(256)
-gemv_batch_kernel(const double* __restrict__ tiles, int ts, int k, const long long* __restrict__ tile_base,
-                  const int* __restrict__ ntv, double* __restrict__ z, const long long* __restrict__ loc_base) {
-  const int p = blockIdx.z;
-  const int i = k + 1 + blockIdx.y;
-  if (i >= ntv[p]) return;
-  double* zp = z + loc_base[p];
-  gemv_panel_body(tiles + (tile_base[p] + tile_slot(i, k, ntv[p])) * (long long)ts * ts, ts,
-                  zp + (long long)k * ts, zp + (long long)i * ts, blockIdx.x);
 }
 
 __global__ void __launch_bounds__(256)
@@ -135,12 +123,14 @@ struct egs_batch {
   int *h_info = nullptr, *h_err = nullptr;
   GemmDesc* d_jobs = nullptr;
   long long* d_begin = nullptr;
+  double* scratch = nullptr;  // panel scratch of every problem
   struct Launch {
     long long job_off, begin_off;
     int njobs;
     long long total;
+    int cfg;
   };
-  std::vector<Launch> diag_launch, panel_launch, trail_launch;  // indexed by (k, kb) or k
+  std::vector<Launch> panel_launch, trail_launch;  // indexed by (k, outer block) and k
   alignas(64) unsigned char tmap[128];
   cudaStream_t stream = nullptr;
   bool own_stream = false;
@@ -184,7 +174,7 @@ void free_batch(egs_batch* b) {
   if (b->graph) cudaGraphDestroy(b->graph);
   void* dev[] = {b->tiles, b->x, b->y, b->z, b->zcpy, b->partial, b->result, b->info, b->err, b->d_n, b->d_nt,
                  b->d_tile_base, b->d_loc_base, b->d_partial_base, b->d_tinfo, b->d_params, b->d_ktab,
-                 b->d_jobs, b->d_begin};
+                 b->d_jobs, b->d_begin, b->scratch};
   for (void* p : dev) cudaFree(p);
   cudaFreeHost(b->h_params);
   cudaFreeHost(b->h_result);
@@ -222,39 +212,36 @@ int build_jobs(egs_batch* b) {
   const int ts = b->ts;
   std::vector<GemmDesc> jobs;
   std::vector<long long> begin;
-  auto add_launch = [&](std::vector<egs_batch::Launch>& dst, const std::vector<GemmDesc>& js) {
-    egs_batch::Launch L{(long long)jobs.size(), (long long)begin.size(), (int)js.size(), 0};
-    long long acc = 0;
-    for (const GemmDesc& d : js) {
+  auto add_launch = [&](std::vector<egs_batch::Launch>& dst, std::vector<GemmDesc>& js) {
+    egs_batch::Launch L{(long long)jobs.size(), (long long)begin.size(), (int)js.size(), 0, 0};
+    for (const GemmDesc& d : js) L.total += d.total;
+    L.cfg = gemm_tile_shape(L.total);
+    L.total = 0;
+    for (GemmDesc& d : js) {
+      d.cfg = L.cfg;
+      finish_desc(d);
       jobs.push_back(d);
-      begin.push_back(acc);
-      acc += d.total;
+      begin.push_back(L.total);
+      L.total += d.total;
     }
-    begin.push_back(acc);
-    L.total = acc;
+    begin.push_back(L.total);
     dst.push_back(L);
   };
-  const int nkb = ts / kBatchInner;
   for (int k = 0; k < b->nt_max; ++k) {
     const int A = b->active[k];
     const int A1 = (k + 1 < b->nt_max) ? b->active[k + 1] : 0;
+    int KB = 0;  // first column of the current outer block
     for (int kb = 0; kb < ts; kb += kBatchInner) {
+      if (panel_outer_blocks(ts, kb) > 1) continue;
+      const int KE = kb + kBatchInner;
       std::vector<GemmDesc> js;
-      if (kb + kBatchInner < ts) {
-        const int m = ts - kb - kBatchInner;
-        const int r0 = k * ts + kb + kBatchInner;
-        for (int p = 0; p < A; ++p) js.push_back(job_desc(b, p, m, m, kBatchInner, r0, kb, k, r0, kb, k, r0, r0, 1));
-      }
-      add_launch(b->diag_launch, js);
-      js.clear();
-      if (kb + kBatchInner < ts) {
-        const int ncols = ts - kb - kBatchInner;
-        const int brow = k * ts + kb + kBatchInner;
-        for (int p = 0; p < A1; ++p)
-          js.push_back(job_desc(b, p, (b->nt[p] - 1 - k) * ts, ncols, kBatchInner, (k + 1) * ts, kb, k, brow, kb, k,
-                                (k + 1) * ts, brow, 0));
+      if (KE < ts) {
+        const int r0 = k * ts + KE;
+        for (int p = 0; p < A; ++p)
+          js.push_back(job_desc(b, p, b->nt[p] * ts - r0, ts - KE, KE - KB, r0, KB, k, r0, KB, k, r0, r0, 1));
       }
       add_launch(b->panel_launch, js);
+      KB = KE;
     }
     std::vector<GemmDesc> js;
     for (int p = 0; p < A1; ++p) {
@@ -263,7 +250,6 @@ int build_jobs(egs_batch* b) {
       js.push_back(job_desc(b, p, m, m, ts, r0, 0, k, r0, 0, k, r0, r0, 1));
     }
     add_launch(b->trail_launch, js);
-    (void)nkb;
   }
   int rc;
   if ((rc = balloc(b, &b->d_jobs, jobs.size())) || (rc = balloc(b, &b->d_begin, begin.size()))) return rc;
@@ -278,7 +264,7 @@ int build_jobs(egs_batch* b) {
 int launch_jobs(egs_batch* b, const egs_batch::Launch& L) {
   if (L.njobs == 0 || L.total == 0) return EGS_OK;
   ++b->launches_per_eval;
-  return launch_gemm_batched(b->tmap, b->tiles, b->d_jobs + L.job_off, b->d_begin + L.begin_off, L.njobs, L.total,
+  return launch_gemm_batched(b->tmap, b->tiles, L.cfg, b->d_jobs + L.job_off, b->d_begin + L.begin_off, L.njobs, L.total,
                              b->err, b->stream);
 }
 
@@ -299,52 +285,43 @@ int enqueue_batch_eval(egs_batch* b) {
                                                               b->d_params, b->d_ktab, b->d_loc_base, b->d_n);
     ++b->launches_per_eval;
   }
-  int li = 0;
+  static std::once_flag step_attr[64];
+  once_per_device(step_attr, []() {
+    cudaFuncSetAttribute(panel_step_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         panel_step_smem(kStepMaxBlocks - 1));
+  });
+  int li = 0, parity = 0;
+  int pk = 0, pkb = 0, pnb = 0, pactive = 0;  // the step still in its scratch slot
   for (int k = 0; k < b->nt_max; ++k) {
     const int A = b->active[k];
-    const int A1 = (k + 1 < b->nt_max) ? b->active[k + 1] : 0;
-    for (int kb = 0; kb < ts; kb += kBatchInner, ++li) {
-      potrf_batch_kernel<<<A, 256, 0, st>>>(b->tiles, ts, k, kb, b->d_tile_base, b->d_nt, b->info);
+    for (int kb = 0; kb < ts; kb += kBatchInner) {
+      const int nb = panel_outer_blocks(ts, kb) - 1;
+      const int steps = std::max(1, ((b->nt_max - k) * ts - kb) / kStep - 1);
+      panel_step_batch_kernel<<<dim3(steps + (pactive ? 1 + pnb : 0), std::max(A, pactive)), kStepThreads,
+                                panel_step_smem(nb), st>>>(b->tiles, ts, k, kb, nb, steps, A, pk, pkb, pnb, pactive,
+                                                           parity, b->d_tile_base, b->d_nt, b->info, b->z,
+                                                           b->d_loc_base, b->scratch);
       ++b->launches_per_eval;
-      if (kb + kBatchInner < ts) {
-        const int rows = ts - kb - kBatchInner;
-        trsm_batch_kernel<<<dim3((rows + 127) / 128, 1, A), 128, 0, st>>>(b->tiles, ts, k, kb + kBatchInner, kb, 0,
-                                                                          b->d_tile_base, b->d_nt);
-        ++b->launches_per_eval;
-        int rc = launch_jobs(b, b->diag_launch[li]);
+      pk = k;
+      pkb = kb;
+      pnb = nb;
+      pactive = A;
+      parity ^= 1;
+      if (nb == 0) {
+        const int rc = launch_jobs(b, b->panel_launch[li++]);
         if (rc != EGS_OK) return rc;
       }
     }
-    li -= ts / kBatchInner;
-    if (A1 > 0) {
-      for (int kb = 0; kb < ts; kb += kBatchInner, ++li) {
-        trsm_batch_kernel<<<dim3((ts + 127) / 128, b->nt_max - k - 1, A1), 128, 0, st>>>(b->tiles, ts, k, 0, kb, 1,
-                                                                                           b->d_tile_base, b->d_nt);
-        ++b->launches_per_eval;
-        int rc = launch_jobs(b, b->panel_launch[li]);
-        if (rc != EGS_OK) return rc;
-      }
-      int rc = launch_jobs(b, b->trail_launch[k]);
-      if (rc != EGS_OK) return rc;
-    } else {
-      li += ts / kBatchInner;
-    }
+    const int rc = launch_jobs(b, b->trail_launch[k]);
+    if (rc != EGS_OK) return rc;
   }
+  panel_step_batch_kernel<<<dim3(1 + pnb, pactive), kStepThreads, 0, st>>>(
+      b->tiles, ts, 0, 0, 0, 0, 0, pk, pkb, pnb, pactive, parity, b->d_tile_base, b->d_nt, b->info, b->z,
+      b->d_loc_base, b->scratch);
+  ++b->launches_per_eval;
   logdet_batch_kernel<<<dim3(b->nt_max, b->B), 256, 0, st>>>(b->tiles, ts, b->d_tile_base, b->d_nt, b->d_n,
                                                              b->partial, b->d_partial_base);
   ++b->launches_per_eval;
-  for (int k = 0; k < b->nt_max; ++k) {
-    const int A = b->active[k];
-    const int A1 = (k + 1 < b->nt_max) ? b->active[k + 1] : 0;
-    trsv_batch_kernel<<<A, 1024, ts * sizeof(double), st>>>(b->tiles, ts, k, b->d_tile_base, b->d_nt, b->z,
-                                                            b->d_loc_base);
-    ++b->launches_per_eval;
-    if (A1 > 0) {
-      gemv_batch_kernel<<<dim3(ts / kBatchInner, b->nt_max - k - 1, A1), 256, ts * sizeof(double), st>>>(
-          b->tiles, ts, k, b->d_tile_base, b->d_nt, b->z, b->d_loc_base);
-      ++b->launches_per_eval;
-    }
-  }
   finalize_batch_kernel<<<b->B, 256, 0, st>>>(b->partial, b->d_partial_base, b->d_nt, b->z, b->d_loc_base, b->d_n,
                                               b->result, b->info);
   ++b->launches_per_eval;
@@ -432,7 +409,8 @@ int egs_batch_create(egs_batch** out, int B, const int* n, int dts, const double
       (rc = balloc(b, &b->d_n, B)) || (rc = balloc(b, &b->d_nt, B)) || (rc = balloc(b, &b->d_tile_base, B)) ||
       (rc = balloc(b, &b->d_loc_base, B)) || (rc = balloc(b, &b->d_partial_base, B)) ||
       (rc = balloc(b, &b->d_tinfo, tinfo.size())) || (rc = balloc(b, &b->d_params, B)) ||
-      (rc = balloc(b, &b->d_ktab, (size_t)B * kKtabDoubles))) {
+      (rc = balloc(b, &b->d_ktab, (size_t)B * kKtabDoubles)) ||
+      (rc = balloc(b, &b->scratch, (size_t)B * kScratchDoubles))) {
     free_batch(b);
     return rc;
   }

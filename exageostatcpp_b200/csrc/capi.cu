@@ -331,7 +331,7 @@ void free_problem(egs_problem* p) {
 // last step's solved rows stay in ch's scratch until the next step or
 // launch_panel_flush.  Returns the launch count in *nl.
 int enqueue_panel(double* tiles, const void* tmap, int ts, int nt, int row_tiles, int k, int col_base, int* info,
-                  int* err, double* z, PanelChain& ch, cudaStream_t st, long long* nl, int max_ctas = 0) {
+                  int* err, double* z, PanelChain& ch, cudaStream_t st, long long* nl) {
   double* col = tiles + tile_slot(k, k, nt) * (long long)ts * ts;
   const int drow = k * ts;
   const int row_end = row_tiles * ts;  // end of the panel's global rows
@@ -346,7 +346,7 @@ int enqueue_panel(double* tiles, const void* tmap, int ts, int nt, int row_tiles
     if (KE < ts) {
       const int r0 = drow + KE;
       rc = launch_gemm_rows(tmap, tiles, ts, nt, row_end - r0, ts - KE, KE - KB, r0, KB, k, r0, KB, k, r0, r0, 1, err,
-                            st, max_ctas);
+                            st);
       if (rc != EGS_OK) return rc;
       ++*nl;
     }
@@ -614,7 +614,7 @@ static int enqueue_short_panel(egs_problem* p, int k, cudaStream_t s, int max_ct
   PanelChain ch;
   ch.scratch = p->pscratch;
   if (int rc = enqueue_panel(p->W2, p->tmapW2, ts, nb + 2, nb + 2, 0, k * ts, p->flags, p->flags + 1, nullptr, ch, s,
-                             &nl, max_ctas))
+                             &nl))
     return rc;
   if (int rc = launch_panel_flush(ch, s)) return rc;
   ++nl;
@@ -732,7 +732,7 @@ int enqueue_eval_mixed(egs_problem* p) {
     sp = span_begin(p, EGS_STAGE_UPDATE);
     const egs_problem::JobLaunch& L = p->band_launch[k];
     if (L.njobs > 0 && L.total > 0) {
-      int rc = launch_gemm_batched(p->tmapW, p->band_pool, p->band_jobs + L.job_off, p->band_begin + L.begin_off,
+      int rc = launch_gemm_batched(p->tmapW, p->band_pool, 0, p->band_jobs + L.job_off, p->band_begin + L.begin_off,
                                    L.njobs, L.total, err, st);
       if (rc != EGS_OK) return rc;
       count_launches(p, EGS_STAGE_UPDATE, 1);

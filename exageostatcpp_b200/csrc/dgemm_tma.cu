@@ -2,24 +2,34 @@
 // fed by TMA, for sm_100a.
 //
 // This is the trailing syrk/gemm of the tiled Cholesky (the N^3/3 part of
-// CHAMELEON_dpotrf_Tile, ChameleonDense.cpp:25-37) and, with K = 64, the
-// updates inside the panel factorisation and the panel triangular solve.
+// CHAMELEON_dpotrf_Tile, ChameleonDense.cpp:25-37) and, with K = 64 or 128, the
+// updates between the outer blocks of a panel.
 //
 // Geometry.  Every operand row is a *global* matrix row g in [0, Np); its data
 // lives in tile row g / ts at local row g % ts.  A and B take their K columns
 // from one tile column (a_tcol / b_tcol) starting at a local column offset; C is
 // addressed element by element through (global row, global column) and
 // elements of upper tiles are never written.  Because ts is a multiple of 64,
-// a 16-row TMA box never straddles two tiles, so a 128 x 128 CTA tile may span
-// tile boundaries and no MMA work is wasted when 128 does not divide ts.
+// a 16-row TMA box never straddles two tiles, so a CTA tile may span tile
+// boundaries.
 //
-// Pipeline.  Thread 0 issues 3-D TMA loads (rows x cols x tile-slot), running up to
-// two stages ahead, into a 3-stage ring of 32-column 128B-swizzled shared-memory
-// stages guarded by mbarriers; eight warps each own a 64 x 32 sub-tile and run
-// mma.sync m16n8k16 .f64 (the FP64 tensor path of sm_100a).  The 16 rows of an
-// MMA fragment are mapped to tile rows through fixed permutations chosen so
-// that every fragment load is free of shared-memory bank conflicts under the
-// 128-byte swizzle (A: 16-byte loads of row pairs; B: 8-byte loads).
+// Work unit.  One CTA computes one C tile (64 x 64, smaller where that would leave
+// SMs idle, gemm_tile_shape) and exits; four CTAs share an SM, so one tile's C
+// round trip and pipeline fill run beside the other tiles' MMAs, and the
+// hardware balances the triangular tile set.  FP64-tensor bound: 33.5 TF/s on the
+// N = 40,000 trailing updates (K = 960; cuBLAS DGEMM about 35.4) and 27.3 at
+// N = 10,000; one persistent 128 x 128 CTA per SM (its epilogue uncovered, whole
+// tiles as the unit of the last wave) reached 27.9 and 20.3, 128 x 64 tiles at two
+// CTAs per SM 31.6 and 25.2.
+//
+// Pipeline.  Warp 0 issues 3-D TMA loads (16 rows x 16 columns x tile-slot, one box
+// per lane) two stages ahead into a ring of 16-column 128B-swizzled shared-memory
+// stages guarded by mbarriers; the four warps, one per SM sub-partition, run
+// mma.sync m16n8k16 .f64 (the FP64 tensor path of sm_100a: one warp keeps its
+// sub-partition's pipe full, 128 cycles per instruction).  The 16 rows of an MMA
+// fragment are mapped to tile rows through fixed permutations chosen so that
+// every fragment load is free of shared-memory bank conflicts under the 128-byte
+// swizzle (A: 16-byte loads of row pairs; B: 8-byte loads).
 //
 // Every wait is bounded: a thread that polls longer than the limit records an
 // error in *err and leaves; the host turns that into EGS_ERR_TIMEOUT.
@@ -34,22 +44,27 @@
 namespace egs {
 
 namespace gemm {
-#ifndef EGS_GEMM_BK
-#define EGS_GEMM_BK 32
-#endif
-#ifndef EGS_GEMM_STAGES
-#define EGS_GEMM_STAGES 3
-#endif
-constexpr int BM = 128, BN = 128, BK = EGS_GEMM_BK, STAGES = EGS_GEMM_STAGES;
-constexpr int CONSUMER_WARPS = 8;
-constexpr int THREADS = CONSUMER_WARPS * 32;   // thread 0 also issues the TMA loads
+constexpr int BK = 16;                                // columns per stage = one MMA k-step
+constexpr int WARPS = 4;                              // 2 x 2 warp tiles; warp 0 also issues the TMA loads
+constexpr int THREADS = WARPS * 32;
+constexpr int LEAD = 2;                               // stages issued ahead of the one being consumed
 constexpr int BOX_ROWS = 16;                          // 16 doubles = one 128-byte swizzle row
 constexpr int BOX_BYTES = BOX_ROWS * BK * 8;          // 16 rows x BK columns
-constexpr int A_STAGE_BYTES = (BM / BOX_ROWS) * BOX_BYTES;
-constexpr int B_STAGE_BYTES = (BN / BOX_ROWS) * BOX_BYTES;
-constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 2 * STAGES * 8 + 1024;
-constexpr int GROUP = 8;                              // block-columns per raster group
+constexpr int GROUP_COLS = 1024;                      // columns per raster group
+
+// Tile shape (GemmDesc::cfg): 0 = 64 x 64, 1 = 64 x 32, 2 = 32 x 32.
+__host__ __device__ constexpr int block_m(int cfg) { return cfg == 2 ? 32 : 64; }
+__host__ __device__ constexpr int block_n(int cfg) { return cfg == 0 ? 64 : 32; }
+template <int CFG>
+struct Shape {
+  static constexpr int BM = block_m(CFG), BN = block_n(CFG);
+  static constexpr int STAGES = CFG == 0 ? 3 : 4;
+  static constexpr int CTAS = 4;                      // per SM, at most 128 registers per thread
+  static constexpr int MI = BM / 32, NI = BN / 16;    // 16 x 8 MMA tiles per warp
+  static constexpr int BOXES = (BM + BN) / BOX_ROWS;
+  static constexpr int STAGE_BYTES = BOXES * BOX_BYTES;
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 2 * STAGES * 8 + 1024;
+};
 }  // namespace gemm
 
 // MMA row g (0..7) of an A fragment -> tile row 2*perm[g] within a 16-row box;
@@ -60,174 +75,131 @@ __device__ __forceinline__ int perm_b(int r) {
   return (r & 1) | (((r >> 2) & 1) << 1) | (((r >> 1) & 1) << 3) | (((r >> 3) & 1) << 2);
 }
 
-template <bool kBatched>
-__device__ __forceinline__ const GemmDesc* locate_job(long long L, const GemmDesc& single, const GemmJobs& J,
-                                                      long long& local) {
-  if constexpr (!kBatched) {
-    local = L;
-    return &single;
-  } else {
-    int lo = 0, hi = J.njobs - 1;
-    while (lo < hi) {  // last job with begin <= L
-      const int mid = (lo + hi + 1) >> 1;
-      if (J.begin[mid] <= L) lo = mid; else hi = mid - 1;
-    }
-    local = L - J.begin[lo];
-    return J.jobs + lo;
-  }
+// Raster: groups of GROUP_COLS columns; inside a group, block-rows outer,
+// block-columns inner, so a group's B panel stays in L2 while A streams once.
+// A lower problem's group starts at the first block-row that reaches its columns.
+__host__ __device__ inline int group_first_row(const GemmDesc& d, int nb0) {
+  return d.lower ? nb0 * gemm::block_n(d.cfg) / gemm::block_m(d.cfg) : 0;
 }
 
-// Raster: groups of GROUP block-columns; inside a group, block-rows outer,
-// block-columns inner, so a group's B panel stays in L2 while A streams once.
-__device__ __forceinline__ bool decode_block(long long L, const GemmDesc& d, int& mb, int& nb) {
-  for (int nb0 = 0; nb0 < d.NB; nb0 += gemm::GROUP) {
-    const int ge = min(gemm::GROUP, d.NB - nb0);
-    const int mstart = d.lower ? nb0 : 0;
+__device__ __forceinline__ void decode_block(long long L, const GemmDesc& d, int& mb, int& nb) {
+  const int group = gemm::GROUP_COLS / gemm::block_n(d.cfg);
+  mb = d.MB;
+  nb = d.NB;
+  for (int nb0 = 0; nb0 < d.NB; nb0 += group) {
+    const int ge = min(group, d.NB - nb0);
+    const int mstart = group_first_row(d, nb0);
     const long long cnt = (long long)ge * (d.MB - mstart);
     if (L < cnt) {
       mb = mstart + (int)(L / ge);
       nb = nb0 + (int)(L % ge);
-      return true;
+      return;
     }
     L -= cnt;
   }
-  return false;
 }
 
 // Blocks with nothing to write: above the diagonal, or (band targets of the
 // lower pool, c_mode 2) wholly below the band.
 __device__ __forceinline__ bool block_skipped(const GemmDesc& d, int mb, int nb) {
-  if (d.lower && mb < nb) return true;
+  const int bm = gemm::block_m(d.cfg), bn = gemm::block_n(d.cfg);
+  if (mb >= d.MB || nb >= d.NB) return true;
+  if (d.lower && (mb + 1) * bm <= nb * bn) return true;
   if (d.c_mode != 2) return false;
-  const int ti = (d.c_row0 + mb * gemm::BM) / d.ts, tj = (d.c_col0 + nb * gemm::BN + gemm::BN - 1) / d.ts;
+  const int ti = (d.c_row0 + mb * bm) / d.ts, tj = (d.c_col0 + nb * bn + bn - 1) / d.ts;
   return ti - tj > d.c_band;
 }
 
-// Producer cursor: walks the same (block, k-step) sequence as the consumers,
-// running up to STAGES-1 stages ahead of them.  The TMA (x, z) coordinates of
-// the 2 x 8 boxes of a block depend only on the block, so they are computed
-// once per block into shared memory; a stage then only adds its k offset.
-struct Cursor {
-  long long L;
-  int kt;
-  bool valid;
-  const GemmDesc* d;
-};
-
-__device__ __forceinline__ void box_coords(int g0, int tcol, const GemmDesc& d, int2* out) {
-#pragma unroll
-  for (int b = 0; b < gemm::BM / gemm::BOX_ROWS; ++b) {
-    const int g = g0 + b * gemm::BOX_ROWS;
-    int x = d.ts, z = 0;  // fully out of bounds -> zero fill
-    if (g < d.np) {
-      const int ti = g / d.ts;
-      x = g - ti * d.ts;
-      z = (int)(d.tile_base + tile_slot(ti, tcol, d.nt));
-    }
-    out[b] = make_int2(x, z);
-  }
+// C(gi, gj) sits at row part + column part: tiles of one column are contiguous.
+__device__ __forceinline__ long long c_row_part(const GemmDesc& d, int gi, int& ti) {
+  ti = gi / d.ts;
+  return (long long)ti * d.ts * d.ts + (gi - ti * d.ts);
+}
+__device__ __forceinline__ long long c_col_part(const GemmDesc& d, int gj, int& tj) {
+  tj = gj / d.ts;
+  const long long slot0 = d.c_mode != 1 ? d.tile_base + tile_slot(tj, tj, d.nt) - tj
+                                        : (long long)(d.c_tile_off + tj) * (d.c_band + 1) - tj;
+  return slot0 * d.ts * d.ts + (long long)(gj - tj * d.ts) * d.ts;
+}
+__device__ __forceinline__ bool c_written(const GemmDesc& d, int ti, int tj) {
+  return ti >= tj && (d.c_mode == 0 || ti - tj <= d.c_band);
 }
 
-template <bool kBatched>
-__device__ __forceinline__ void cursor_seek(Cursor& c, const GemmDesc& single, const GemmJobs& J, long long total,
-                                            int2* coords) {
-  while (c.L < total) {
-    long long local;
-    const GemmDesc& d = *locate_job<kBatched>(c.L, single, J, local);
-    int mb, nb;
-    decode_block(local, d, mb, nb);
-    if (!block_skipped(d, mb, nb)) {
-      box_coords(d.a_row0 + mb * gemm::BM, d.a_tcol, d, coords);
-      box_coords(d.b_row0 + nb * gemm::BN, d.b_tcol, d, coords + gemm::BM / gemm::BOX_ROWS);
-      c.d = &d;
-      c.valid = true;
-      return;
-    }
-    c.L += gridDim.x;
-  }
-  c.valid = false;
-}
-
-__device__ __forceinline__ void issue_stage(const CUtensorMap* tmap, uint8_t* smem, uint64_t* full, uint32_t s,
-                                            const Cursor& c, const int2* coords) {
+template <int CFG, bool kBatched>
+__global__ void __launch_bounds__(gemm::THREADS, gemm::Shape<CFG>::CTAS)
+dgemm_update_kernel(const __grid_constant__ CUtensorMap tmap, double* __restrict__ tiles,
+                    const __grid_constant__ GemmDesc single, GemmJobs J, int* __restrict__ err) {
   using namespace gemm;
-  const GemmDesc& d = *c.d;
-  mbar_expect_tx(&full[s], STAGE_BYTES);
-  uint8_t* sa = smem + s * STAGE_BYTES;
-  uint8_t* sb = sa + A_STAGE_BYTES;
-  const int ya = d.a_col0 + c.kt * BK, yb = d.b_col0 + c.kt * BK;
-#pragma unroll
-  for (int b = 0; b < BM / BOX_ROWS; ++b) {
-    const int2 xz = coords[b];
-    tma_load_3d(sa + b * BOX_BYTES, tmap, &full[s], xz.x, ya, xz.y);
-  }
-#pragma unroll
-  for (int b = 0; b < BN / BOX_ROWS; ++b) {
-    const int2 xz = coords[BM / BOX_ROWS + b];
-    tma_load_3d(sb + b * BOX_BYTES, tmap, &full[s], xz.x, yb, xz.y);
-  }
-}
-
-template <bool kBatched>
-__global__ void __launch_bounds__(gemm::THREADS, 1)
-dgemm_update_kernel(const __grid_constant__ CUtensorMap tmap, double* __restrict__ tiles, const __grid_constant__ GemmDesc single,
-                    GemmJobs J, int* __restrict__ err) {
-  using namespace gemm;
+  using S = Shape<CFG>;
+  constexpr int BM = S::BM, BN = S::BN, STAGES = S::STAGES;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
+  // the job of this block, and its tile
+  const GemmDesc* dp = &single;
+  long long L = blockIdx.x;
+  if constexpr (kBatched) {
+    int lo = 0, hi = J.njobs - 1;
+    while (lo < hi) {  // last job with begin <= L
+      const int mid = (lo + hi + 1) >> 1;
+      if (J.begin[mid] <= L) lo = mid; else hi = mid - 1;
+    }
+    L -= J.begin[lo];
+    dp = J.jobs + lo;
+  }
+  const GemmDesc& d = *dp;
+  int mb, nb;
+  decode_block(L, d, mb, nb);
+  if (block_skipped(d, mb, nb)) return;
   // 1024-byte aligned stage base (128B-swizzle atoms), kept as an offset into the
   // shared array so every access stays a shared-memory access.
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  const uint32_t smem_s = smem_u32(smem);
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * S::STAGE_BYTES);
   uint64_t* empty = full + STAGES;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const bool producer = threadIdx.x == 0;
-  const long long total = kBatched ? J.total : single.total;
-  if (producer) {
+  if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&full[s], 1);
-      mbar_init(&empty[s], CONSUMER_WARPS);
+      mbar_init(&empty[s], WARPS);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)&tmap) : "memory");
   }
   __syncthreads();
+  const int ksteps = d.K / BK;
 
-  // Producer state (meaningful in thread 0 only).
-  __shared__ int2 coords[(BM + BN) / BOX_ROWS];
-  Cursor cur;
-  cur.L = blockIdx.x;
-  cur.kt = 0;
-  cur.valid = false;
-  uint32_t issued = 0;
-  bool alive = true;
-  cur.d = &single;
-  if (producer) cursor_seek<kBatched>(cur, single, J, total, coords);
-  auto top_up = [&](uint32_t consumed) {
-    // Keep up to STAGES-1 stages in flight ahead of the consumers.
-    while (alive && cur.valid && issued < consumed + STAGES - 1) {
-      const uint32_t s = issued % STAGES, ph = (issued / STAGES) & 1;
-      if (!mbar_wait(&empty[s], ph ^ 1, err)) {
-        alive = false;
-        break;
-      }
-      issue_stage(&tmap, smem, full, s, cur, coords);
-      ++issued;
-      if (++cur.kt == cur.d->K / BK) {
-        cur.kt = 0;
-        cur.L += gridDim.x;
-        cursor_seek<kBatched>(cur, single, J, total, coords);
-      }
+  // Producer state: lane b of warp 0 loads box b of every stage (A boxes first).
+  int x = d.ts, z = 0, y0 = 0;  // fully out of bounds -> zero fill
+  if (warp == 0 && lane < S::BOXES) {
+    const bool is_a = lane < BM / BOX_ROWS;
+    const int g0 = is_a ? d.a_row0 + mb * BM + lane * BOX_ROWS : d.b_row0 + nb * BN + (lane - BM / BOX_ROWS) * BOX_ROWS;
+    y0 = is_a ? d.a_col0 : d.b_col0;
+    if (g0 < d.np) {
+      const int tg = g0 / d.ts;
+      x = g0 - tg * d.ts;
+      z = (int)(d.tile_base + tile_slot(tg, is_a ? d.a_tcol : d.b_tcol, d.nt));
     }
+  }
+  // Issues stage j (warp 0, all lanes); its slot was last used by stage j - STAGES.
+  auto issue = [&](int j) {
+    const int sj = j % STAGES;
+    bool slot_free = true;
+    if (lane == 0) {
+      slot_free = mbar_wait(&empty[sj], ((j / STAGES) & 1) ^ 1, err);
+      if (slot_free) mbar_expect_tx(&full[sj], S::STAGE_BYTES);
+    }
+    if (!__shfl_sync(0xffffffffu, (int)slot_free, 0)) return false;
+    if (lane < S::BOXES)
+      tma_load_3d(smem + sj * S::STAGE_BYTES + lane * BOX_BYTES, &tmap, &full[sj], x, y0 + j * BK, z);
+    return true;
   };
+  int issued = 0;  // stages whose copies are under way (warp 0)
+  if (warp == 0)
+    while (issued < min(LEAD, ksteps) && issue(issued)) ++issued;
 
   const int g = lane >> 2, t = lane & 3;
-  const int wm = warp & 1, wn = warp >> 1;  // warp sub-tile: rows wm*64.., cols wn*32..
+  const int wm = warp & 1, wn = warp >> 1;  // warp sub-tile: rows wm*BM/2.., cols wn*BN/2..
   const int pa = perm_a(g);
-  const int row_in_box = 2 * pa;  // accumulator rows row_in_box, row_in_box + 1
   // Byte offsets (inside one 16-row box) of this thread's fragment elements.
-  uint32_t aoff[4], boff[2][4];
+  int aoff[4], boff[2][4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     const int k = t + 4 * j;
@@ -242,97 +214,102 @@ dgemm_update_kernel(const __grid_constant__ CUtensorMap tmap, double* __restrict
       boff[sN][i] = k * 128 + (((fb >> 1) ^ (k & 7)) << 4) + ((fb & 1) << 3);
     }
   }
-
-  uint32_t it = 0;
-  bool ok = true;
-  for (long long L = blockIdx.x; L < total && ok; L += gridDim.x) {
-    long long local;
-    const GemmDesc& d = *locate_job<kBatched>(L, single, J, local);
-    int mb, nb;
-    decode_block(local, d, mb, nb);
-    if (block_skipped(d, mb, nb)) continue;
-    const int ksteps = d.K / BK;
-    double acc[4][4][4];
+  {
+    // this warp's part of C to L2: one column per lane, 16 rows (128 bytes) per request
+    const int nl = nb * BN + wn * (BN / 2) + (lane & (BN / 2 - 1));
+    int tj;
+    const long long cp = c_col_part(d, d.c_col0 + nl, tj);
 #pragma unroll
-    for (int mi = 0; mi < 4; ++mi)
-#pragma unroll
-      for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) acc[mi][ni][q] = 0.0;
-
-    for (int kt = 0; kt < ksteps; ++kt, ++it) {
-      if (producer) top_up(it);
-      __syncwarp();
-      const uint32_t s = it % STAGES, ph = (it / STAGES) & 1;
-      if (!mbar_wait(&full[s], ph, err)) {
-        ok = false;
-        break;
-      }
-      __syncwarp();
-      const uint32_t sa = smem_s + s * STAGE_BYTES;
-      const uint32_t sb = sa + A_STAGE_BYTES;
-#pragma unroll
-      for (int kk = 0; kk < BK / 16; ++kk) {
-        const uint32_t koff = kk * 16 * 128;  // 16 k-rows of 128 bytes per MMA k-step
-        double bf[4][4];
-#pragma unroll
-        for (int ni = 0; ni < 4; ++ni) {
-          const uint32_t box = sb + (wn * 2 + (ni >> 1)) * BOX_BYTES + koff;
-#pragma unroll
-          for (int i = 0; i < 4; ++i) bf[ni][i] = lds_f64(box + boff[ni & 1][i]);
-        }
-#pragma unroll
-        for (int mi = 0; mi < 4; ++mi) {
-          const uint32_t box = sa + (wm * 4 + mi) * BOX_BYTES + koff;
-          double af[8];
-#pragma unroll
-          for (int j = 0; j < 4; ++j) lds_v2f64(box + aoff[j], af[2 * j], af[2 * j + 1]);
-#pragma unroll
-          for (int ni = 0; ni < 4; ++ni) dmma_16816(acc[mi][ni], af, bf[ni]);
-        }
-      }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&empty[s]);
-    }
-    if (!ok) break;
-
-    // Epilogue: C -= acc; element pairs (row, row+1) are contiguous in a column.
-    // Per n8 block the eight 16-byte loads are issued before any store, so a
-    // thread pays one memory round trip per block instead of one per pair.
-    const int ts = d.ts;
-#pragma unroll
-    for (int ni = 0; ni < 4; ++ni) {
-      double* ptr[2][4];
-      double cv[2][4][2];
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int nl = nb * BN + wn * 32 + (ni >> 1) * 16 + perm_b(2 * t + 8 * (ni & 1)) + h;
-        const int gj = d.c_col0 + nl;
-        const int tj = gj / ts, lc = gj - tj * ts;
-#pragma unroll
-        for (int mi = 0; mi < 4; ++mi) {
-          const int ml = mb * BM + wm * 64 + mi * 16 + row_in_box;
-          const int gi = d.c_row0 + ml;
-          const int ti = gi / ts, lr = gi - ti * ts;
-          const bool ok_el = nl < d.N && ml < d.M && ti >= tj && (d.c_mode == 0 || ti - tj <= d.c_band);
-          const long long cslot = d.c_mode != 1 ? d.tile_base + tile_slot(ti, tj, d.nt)
-                                                : (long long)(d.c_tile_off + tj) * (d.c_band + 1) + (ti - tj);
-          ptr[h][mi] = ok_el ? tiles + cslot * (long long)ts * ts + (long long)lc * ts + lr : nullptr;
-          if (ok_el) ldg_v2f64(ptr[h][mi], cv[h][mi][0], cv[h][mi][1]);
-        }
-      }
-#pragma unroll
-      for (int h = 0; h < 2; ++h)
-#pragma unroll
-        for (int mi = 0; mi < 4; ++mi)
-          if (ptr[h][mi])
-            stg_v2f64(ptr[h][mi], cv[h][mi][0] - acc[mi][ni][h], cv[h][mi][1] - acc[mi][ni][2 + h]);
+    for (int mi = 0; mi < S::MI; ++mi) {
+      const int ml = mb * BM + wm * (BM / 2) + mi * 16;
+      int ti;
+      const long long p = c_row_part(d, d.c_row0 + ml, ti) + cp;
+      if (nl < d.N && ml < d.M && c_written(d, ti, tj)) asm volatile("prefetch.global.L2 [%0];" ::"l"(tiles + p));
     }
   }
-  // Drain: every stage this CTA issued must have landed before it exits.
-  if (producer) {
-    for (uint32_t j = (issued > (uint32_t)STAGES ? issued - STAGES : 0); j < issued; ++j)
-      mbar_wait(&full[j % STAGES], (j / STAGES) & 1, err);
+  double acc[S::MI][S::NI][4];
+#pragma unroll
+  for (int mi = 0; mi < S::MI; ++mi)
+#pragma unroll
+    for (int ni = 0; ni < S::NI; ++ni)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) acc[mi][ni][q] = 0.0;
+
+  bool ok = true;
+  int s = 0, ph = 0;
+#pragma unroll 1
+  for (int kt = 0; kt < ksteps; ++kt) {
+    if (warp == 0 && kt + LEAD < ksteps && issued == kt + LEAD && issue(issued)) ++issued;
+    if (!mbar_wait(&full[s], ph, err)) {
+      ok = false;
+      break;
+    }
+    const uint8_t* sa = smem + s * S::STAGE_BYTES + wm * (BM / 2 / BOX_ROWS) * BOX_BYTES;
+    const uint8_t* sb = smem + s * S::STAGE_BYTES + (BM / BOX_ROWS + wn * (BN / 2 / BOX_ROWS)) * BOX_BYTES;
+    double bf[S::NI][4];
+#pragma unroll
+    for (int ni = 0; ni < S::NI; ++ni)
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        bf[ni][i] = *reinterpret_cast<const double*>(sb + (ni >> 1) * BOX_BYTES + boff[ni & 1][i]);
+#pragma unroll
+    for (int mi = 0; mi < S::MI; ++mi) {
+      double af[8];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const double2 v = *reinterpret_cast<const double2*>(sa + mi * BOX_BYTES + aoff[j]);
+        af[2 * j] = v.x;
+        af[2 * j + 1] = v.y;
+      }
+#pragma unroll
+      for (int ni = 0; ni < S::NI; ++ni) dmma_16816(acc[mi][ni], af, bf[ni]);
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&empty[s]);
+    if (++s == STAGES) {
+      s = 0;
+      ph ^= 1;
+    }
+  }
+  if (!ok) {
+    // Drain: every stage this CTA issued must have landed before it exits.
+    if (threadIdx.x == 0)
+      for (int j = (issued > STAGES ? issued - STAGES : 0); j < issued; ++j)
+        mbar_wait(&full[j % STAGES], (j / STAGES) & 1, err);
+    return;
+  }
+
+  // Epilogue: C -= acc; element pairs (row, row+1) are contiguous in a column.
+  // Per n8 block all loads are issued before any store.
+  long long rp[S::MI];
+  int ti[S::MI];
+#pragma unroll
+  for (int mi = 0; mi < S::MI; ++mi) {
+    const int ml = mb * BM + wm * (BM / 2) + mi * 16 + 2 * pa;
+    rp[mi] = c_row_part(d, d.c_row0 + ml, ti[mi]);
+    if (ml >= d.M) ti[mi] = -1;  // above every tile column: not written
+  }
+#pragma unroll
+  for (int ni = 0; ni < S::NI; ++ni) {
+    double* ptr[2][S::MI];
+    double cv[2][S::MI][2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int nl = nb * BN + wn * (BN / 2) + (ni >> 1) * 16 + perm_b(2 * t + 8 * (ni & 1)) + h;
+      int tj;
+      const long long cp = c_col_part(d, d.c_col0 + nl, tj);
+#pragma unroll
+      for (int mi = 0; mi < S::MI; ++mi) {
+        ptr[h][mi] = (nl < d.N && c_written(d, ti[mi], tj)) ? tiles + (rp[mi] + cp) : nullptr;
+        if (ptr[h][mi]) ldg_v2f64(ptr[h][mi], cv[h][mi][0], cv[h][mi][1]);
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int mi = 0; mi < S::MI; ++mi)
+        if (ptr[h][mi])
+          stg_v2f64(ptr[h][mi], cv[h][mi][0] - acc[mi][ni][h], cv[h][mi][1] - acc[mi][ni][2 + h]);
   }
 }
 
@@ -389,36 +366,63 @@ int gemm_num_sms() {
 static void set_gemm_smem_attributes() {
   static std::once_flag done[64];
   once_per_device(done, []() {
-    cudaFuncSetAttribute(dgemm_update_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm::SMEM_BYTES);
-    cudaFuncSetAttribute(dgemm_update_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm::SMEM_BYTES);
+    constexpr auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaFuncSetAttribute(dgemm_update_kernel<0, false>, attr, gemm::Shape<0>::SMEM_BYTES);
+    cudaFuncSetAttribute(dgemm_update_kernel<0, true>, attr, gemm::Shape<0>::SMEM_BYTES);
+    cudaFuncSetAttribute(dgemm_update_kernel<1, false>, attr, gemm::Shape<1>::SMEM_BYTES);
+    cudaFuncSetAttribute(dgemm_update_kernel<1, true>, attr, gemm::Shape<1>::SMEM_BYTES);
+    cudaFuncSetAttribute(dgemm_update_kernel<2, false>, attr, gemm::Shape<2>::SMEM_BYTES);
+    cudaFuncSetAttribute(dgemm_update_kernel<2, true>, attr, gemm::Shape<2>::SMEM_BYTES);
   });
+}
+
+// Tile shape of a launch of `total` 64 x 64 tiles.  The large tile reads least from
+// L2 and wins once every SM has four of them (N = 40,000 trailing updates: 33.5
+// TF/s against 32.3 with 64 x 32 and 30.8 with 32 x 32); a smaller launch is
+// bound by the K loop of its one or two tiles per SM, which a smaller tile
+// shortens (band approximation N = 10,000, tile 320, about 340 tiles a launch: 1.16 ms
+// of updates with 64 x 32, 1.47 / 1.29 with the others; N = 1,600, 15 to 210
+// tiles: 104 us with 32 x 32, 115 / 147 with the larger ones).
+int gemm_tile_shape(long long total) {
+  const long long sms = gemm_num_sms();
+  return total < sms ? 2 : total < 4 * sms ? 1 : 0;
 }
 
 void finish_desc(GemmDesc& d) {
   using namespace gemm;
-  d.MB = (d.M + BM - 1) / BM;
-  d.NB = (d.N + BN - 1) / BN;
+  d.MB = (d.M + block_m(d.cfg) - 1) / block_m(d.cfg);
+  d.NB = (d.N + block_n(d.cfg) - 1) / block_n(d.cfg);
+  const int group = GROUP_COLS / block_n(d.cfg);
   long long total = 0;
-  for (int nb0 = 0; nb0 < d.NB; nb0 += GROUP) {
-    const int ge = (d.NB - nb0) < GROUP ? (d.NB - nb0) : GROUP;
-    total += (long long)ge * (d.MB - (d.lower ? nb0 : 0));
+  for (int nb0 = 0; nb0 < d.NB; nb0 += group) {
+    const int ge = (d.NB - nb0) < group ? (d.NB - nb0) : group;
+    total += (long long)ge * (d.MB - group_first_row(d, nb0));
   }
   d.total = total;
 }
 
-static int launch_desc(const void* tmap, double* tiles, GemmDesc& d, int* err, cudaStream_t st, int max_ctas = 0) {
+template <bool kBatched>
+static int launch_cfg(int cfg, const void* tmap, double* tiles, const GemmDesc& d, const GemmJobs& J, long long total,
+                      int* err, cudaStream_t st) {
   using namespace gemm;
-  if (d.M <= 0 || d.N <= 0 || d.K <= 0) return EGS_OK;
-  if (d.K % BK != 0) return EGS_ERR_INVALID;
-  finish_desc(d);
-  const long long total = d.total;
   set_gemm_smem_attributes();
-  const long long cap = (max_ctas > 0 && max_ctas < gemm_num_sms()) ? max_ctas : gemm_num_sms();
-  const long long grid = total < cap ? total : cap;
-  GemmJobs none{nullptr, nullptr, 0, 0};
-  dgemm_update_kernel<false><<<(unsigned)grid, THREADS, SMEM_BYTES, st>>>(
-      *reinterpret_cast<const CUtensorMap*>(tmap), tiles, d, none, err);
+  const CUtensorMap& tm = *reinterpret_cast<const CUtensorMap*>(tmap);
+  if (cfg == 0)
+    dgemm_update_kernel<0, kBatched><<<(unsigned)total, THREADS, Shape<0>::SMEM_BYTES, st>>>(tm, tiles, d, J, err);
+  else if (cfg == 2)
+    dgemm_update_kernel<2, kBatched><<<(unsigned)total, THREADS, Shape<2>::SMEM_BYTES, st>>>(tm, tiles, d, J, err);
+  else
+    dgemm_update_kernel<1, kBatched><<<(unsigned)total, THREADS, Shape<1>::SMEM_BYTES, st>>>(tm, tiles, d, J, err);
   return launch_status("dgemm_update_kernel");
+}
+
+static int launch_desc(const void* tmap, double* tiles, GemmDesc& d, int* err, cudaStream_t st) {
+  if (d.M <= 0 || d.N <= 0 || d.K <= 0) return EGS_OK;
+  if (d.K % gemm::BK != 0) return EGS_ERR_INVALID;
+  d.cfg = 0;
+  finish_desc(d);
+  if ((d.cfg = gemm_tile_shape(d.total)) != 0) finish_desc(d);
+  return launch_cfg<false>(d.cfg, tmap, tiles, d, GemmJobs{nullptr, nullptr, 0, 0}, d.total, err, st);
 }
 
 // Trailing update of step k: C(i, j) -= L(i, k) L(j, k)^T for all k < j <= i.
@@ -461,7 +465,7 @@ int launch_gemm_band(const void* tmap, double* tiles, int ts, int nt, int k, int
 // General form used by the panel factorisation (see kernels.cuh).
 int launch_gemm_rows(const void* tmap, double* tiles, int ts, int nt, int M, int N, int K, int a_row0,
                      int a_col0, int a_tcol, int b_row0, int b_col0, int b_tcol, int c_row0, int c_col0,
-                     int lower, int* err, cudaStream_t st, int max_ctas) {
+                     int lower, int* err, cudaStream_t st) {
   GemmDesc d{};
   d.ts = ts;
   d.nt = nt;
@@ -478,26 +482,20 @@ int launch_gemm_rows(const void* tmap, double* tiles, int ts, int nt, int M, int
   d.c_row0 = c_row0;
   d.c_col0 = c_col0;
   d.lower = lower;
-  return launch_desc(tmap, tiles, d, err, st, max_ctas);
+  return launch_desc(tmap, tiles, d, err, st);
 }
 
 }  // namespace egs
 
 namespace egs {
 
-// One launch over many jobs (one per problem of a batch); jobs and begin live in
-// device memory, begin[j] = number of blocks of jobs 0..j-1 (finish_desc totals).
-int launch_gemm_batched(const void* tmap, double* tiles, const GemmDesc* jobs, const long long* begin, int njobs,
-                        long long total, int* err, cudaStream_t st) {
-  using namespace gemm;
+// One launch over many jobs (one per problem of a batch) of one tile shape cfg;
+// jobs and begin live in device memory, begin[j] = number of blocks of jobs 0..j-1 (finish_desc totals).
+int launch_gemm_batched(const void* tmap, double* tiles, int cfg, const GemmDesc* jobs, const long long* begin,
+                        int njobs, long long total, int* err, cudaStream_t st) {
   if (njobs <= 0 || total <= 0) return EGS_OK;
-  set_gemm_smem_attributes();
-  const long long grid = total < gemm_num_sms() ? total : gemm_num_sms();
   GemmDesc none{};
-  GemmJobs J{jobs, begin, njobs, total};
-  dgemm_update_kernel<true><<<(unsigned)grid, THREADS, SMEM_BYTES, st>>>(
-      *reinterpret_cast<const CUtensorMap*>(tmap), tiles, none, J, err);
-  return launch_status("dgemm_update_kernel (jobs)");
+  return launch_cfg<true>(cfg, tmap, tiles, none, GemmJobs{jobs, begin, njobs, total}, total, err, st);
 }
 
 }  // namespace egs

@@ -76,6 +76,7 @@ struct GemmDesc {
   // ti - tj <= c_band are written, at slot (c_tile_off + tj) * (c_band + 1) + (ti - tj);
   // c_mode 2 = lower-tile pool, only tiles with ti - tj <= c_band.
   int c_mode, c_band, c_tile_off;
+  int cfg;  // tile shape of the launch (dgemm_tma.cu); set before finish_desc
 };
 
 // Batched launches: blocks [begin[j], begin[j+1]) belong to job j.
@@ -87,8 +88,9 @@ struct GemmJobs {
 };
 
 void finish_desc(GemmDesc& d);  // fills MB, NB, total
-int launch_gemm_batched(const void* tmap, double* tiles, const GemmDesc* jobs, const long long* begin, int njobs,
-                        long long total, int* err, cudaStream_t st);
+int gemm_tile_shape(long long total);  // cfg of a launch of `total` blocks of shape 0
+int launch_gemm_batched(const void* tmap, double* tiles, int cfg, const GemmDesc* jobs, const long long* begin,
+                        int njobs, long long total, int* err, cudaStream_t st);
 int gemm_init_tensor_map(void* tmap_storage, double* tiles, int ts, long long ntiles);
 // The driver's cuTensorMapEncodeTiled (looked up once).
 int tensor_map_encoder(void** fn);
@@ -96,7 +98,7 @@ int launch_gemm_trailing(const void* tmap, double* tiles, int ts, int nt, int k,
 int launch_gemm_band(const void* tmap, double* tiles, int ts, int nt, int k, int band, int* err, cudaStream_t st);
 int launch_gemm_rows(const void* tmap, double* tiles, int ts, int nt, int M, int N, int K, int a_row0,
                      int a_col0, int a_tcol, int b_row0, int b_col0, int b_tcol, int c_row0, int c_col0,
-                     int lower, int* err, cudaStream_t st, int max_ctas = 0);
+                     int lower, int* err, cudaStream_t st);
 int gemm_num_sms();
 
 // Mixed-precision evaluation (mixed.cu, split_gemm.cu).

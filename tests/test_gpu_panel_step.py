@@ -45,6 +45,20 @@ def test_factor_and_carried_solve(n, dts, scale):
     p.close()
 
 
+@pytest.mark.parametrize("n,dts", [(1400, 320), (2700, 320), (3001, 960)])
+def test_update_tile_shapes(n, dts):
+    # trailing updates of fewer than 148, 148 to 591 and more 64 x 64 tiles
+    theta = [1.0, 0.03, 0.5]
+    x, y = egs.generate_locations(n, 3)
+    p = egs.Problem(n, dts)
+    p.set_locations(x, y)
+    p.generate(theta)
+    p.potrf()
+    L = np.linalg.cholesky(O.covariance(x, y, theta))
+    assert np.abs(p.lower_matrix() - L).max() <= 1e-10 * np.abs(L).max()
+    p.close()
+
+
 @pytest.mark.parametrize("n,dts,bad", [(300, 320, 0), (300, 320, 63), (300, 320, 64), (300, 320, 201), (700, 192, 390),
                                        (700, 192, 699)])
 def test_failing_pivot_is_reported(n, dts, bad):
