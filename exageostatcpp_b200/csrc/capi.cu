@@ -448,26 +448,24 @@ int enqueue_potrf_band(egs_problem* p) {
   return check_cuda("enqueue_potrf_band");
 }
 
-// Z := L^-1 Z, tile by tile (forward substitution).
-void enqueue_trsv(egs_problem* p) {
+// Z := L^-1 Z (forward substitution).
+int enqueue_trsv(egs_problem* p) {
   const int sp = span_begin(p, EGS_STAGE_SOLVE);
-  for (int k = 0; k < p->nt; ++k) {
-    launch_trsv_diag(p->tiles, p->ts, tile_slot(k, k, p->nt), p->z + (long long)k * p->ts, p->stream);
-    launch_gemv_panel(p->tiles, p->ts, p->nt, k, p->z, p->stream);
-    count_launches(p, EGS_STAGE_SOLVE, k < p->nt - 1 ? 2 : 1);
-  }
+  long long nl = 0;
+  const int rc = launch_vec_forward(p->tiles, p->ts, p->nt, p->z, p->pscratch, p->stream, &nl);
+  count_launches(p, EGS_STAGE_SOLVE, nl);
   span_end(p, sp, (double)p->n * (double)p->n);
+  return rc;
 }
 
 // Z := L^-T Z (backward substitution), the second half of dposv.
-void enqueue_trsv_t(egs_problem* p) {
+int enqueue_trsv_t(egs_problem* p) {
   const int sp = span_begin(p, EGS_STAGE_SOLVE);
-  for (int k = p->nt - 1; k >= 0; --k) {
-    launch_trsv_t_diag(p->tiles, p->ts, tile_slot(k, k, p->nt), p->z + (long long)k * p->ts, p->stream);
-    launch_gemv_t_panel(p->tiles, p->ts, p->nt, k, p->z, p->stream);
-    count_launches(p, EGS_STAGE_SOLVE, k > 0 ? 2 : 1);
-  }
+  long long nl = 0;
+  const int rc = launch_vec_backward(p->tiles, p->ts, p->nt, p->z, p->pscratch, p->stream, &nl);
+  count_launches(p, EGS_STAGE_SOLVE, nl);
   span_end(p, sp, (double)p->n * (double)p->n);
+  return rc;
 }
 
 int set_params(egs_problem* p, const double* theta) {
@@ -525,7 +523,7 @@ int enqueue_eval(egs_problem* p) {
   launch_logdet_partials(p->tiles, p->ts, p->nt, p->n, p->partial, st);
   span_end(p, sp, 0.0);
   count_launches(p, EGS_STAGE_REDUCE, 1);
-  if (p->band > 0) enqueue_trsv(p);
+  if (p->band > 0 && (rc = enqueue_trsv(p)) != EGS_OK) return rc;
   sp = span_begin(p, EGS_STAGE_REDUCE);
   launch_finalize(p->partial, p->nt, p->z, p->n, p->result, p->flags, st);
   span_end(p, sp, 0.0);
@@ -1325,9 +1323,7 @@ int egs_restore_observations(egs_problem* p) {
 int egs_trsv(egs_problem* p) {
   if (!p) return EGS_ERR_INVALID;
   if (int rc = reject_mixed(p, "egs_trsv")) return rc;
-  enqueue_trsv(p);
-  int rc = check_cuda("egs_trsv");
-  if (rc != EGS_OK) return rc;
+  if (int rc = enqueue_trsv(p)) return rc;
   EGS_CUDA_TRY(cudaStreamSynchronize(p->stream));
   return EGS_OK;
 }
@@ -1382,9 +1378,7 @@ int egs_save_observations(egs_problem* p) {
 int egs_trsv_transpose(egs_problem* p) {
   if (!p) return EGS_ERR_INVALID;
   if (int rc = reject_mixed(p, "egs_trsv_transpose")) return rc;
-  enqueue_trsv_t(p);
-  int rc = check_cuda("egs_trsv_transpose");
-  if (rc != EGS_OK) return rc;
+  if (int rc = enqueue_trsv_t(p)) return rc;
   EGS_CUDA_TRY(cudaStreamSynchronize(p->stream));
   return EGS_OK;
 }
@@ -1728,6 +1722,28 @@ int egs_mle_loglik_host(int n, int dts, const double* x, const double* y, const 
   return egs_mle_eval(p, theta, loglik, nullptr, nullptr);
 }
 
+// Z := C(theta)^-1 Zcpy (dposv): generation, factorisation carrying the forward
+// solve, backward solve, one wait.  Positive status: not positive definite (Z
+// holds the observations again then).
+static int posv(egs_problem* p, const double* theta) {
+  int rc = set_params(p, theta);
+  if (rc != EGS_OK) return rc;
+  cudaStream_t st = p->stream;
+  EGS_CUDA_TRY(cudaMemsetAsync(p->flags, 0, 2 * sizeof(int), st));
+  EGS_CUDA_TRY(cudaMemcpyAsync(p->z, p->zcpy, p->np * sizeof(double), cudaMemcpyDeviceToDevice, st));
+  if ((rc = launch_matern_tiles(p->tiles, p->x, p->y, p->n, p->ts, p->nt, p->dparams, p->ktab, st)) != EGS_OK)
+    return rc;
+  if (p->band > 0) {
+    if ((rc = enqueue_potrf_band(p)) != EGS_OK || (rc = enqueue_trsv(p)) != EGS_OK) return rc;
+  } else if ((rc = enqueue_potrf(p, p->z)) != EGS_OK) {
+    return rc;
+  }
+  if ((rc = enqueue_trsv_t(p)) != EGS_OK) return rc;
+  if ((rc = sync_flags(p, false)) != EGS_OK)
+    cudaMemcpyAsync(p->z, p->zcpy, p->np * sizeof(double), cudaMemcpyDeviceToDevice, st);
+  return rc;
+}
+
 int egs_predict_host(int n_obs, int n_miss, int dts, const double* x_obs, const double* y_obs, const double* z_obs,
                      const double* x_miss, const double* y_miss, const double* z_actual, const double* theta,
                      double* z_miss, double* mspe) {
@@ -1740,12 +1756,8 @@ int egs_predict_host(int n_obs, int n_miss, int dts, const double* x_obs, const 
   std::unique_ptr<egs_problem, int (*)(egs_problem*)> guard(p, egs_problem_destroy);
   if ((rc = egs_problem_set_locations(p, x_obs, y_obs)) != EGS_OK) return rc;
   if ((rc = egs_problem_set_observations(p, z_obs)) != EGS_OK) return rc;
-  if ((rc = egs_covariance_generate(p, theta)) != EGS_OK) return rc;
-  if ((rc = egs_potrf(p)) != EGS_OK) return rc;
   // dposv: w = C22^-1 Zobs (LinearAlgebraMethods.cpp:544)
-  enqueue_trsv(p);
-  enqueue_trsv_t(p);
-  if ((rc = check_cuda("egs_predict_host/posv")) != EGS_OK) return rc;
+  if ((rc = posv(p, theta)) != EGS_OK) return rc;
   // C12^T (obs x miss) and Zmiss = C12 w (:535, :552)
   double *c12t = nullptr, *dxm = nullptr, *dym = nullptr, *dzm = nullptr, *dza = nullptr, *dsum = nullptr;
   long long dummy = 0;
@@ -1841,11 +1853,7 @@ int egs_problem_predict(egs_problem* p, const double* theta, int n_miss, const d
     if ((rc = egs_mle_eval(p, theta, &ll, nullptr, nullptr)) != EGS_OK) return rc;
     launch_add_inplace(p->z, p->w, p->n, p->stream);
   } else {
-    if ((rc = egs_covariance_generate(p, theta)) != EGS_OK) return rc;
-    if ((rc = egs_potrf(p)) != EGS_OK) return rc;
-    if ((rc = egs_restore_observations(p)) != EGS_OK) return rc;
-    enqueue_trsv(p);
-    enqueue_trsv_t(p);
+    if ((rc = posv(p, theta)) != EGS_OK) return rc;
   }
   cudaStream_t st = p->stream;
   double *c12t = nullptr, *dxm = nullptr, *dym = nullptr, *dzm = nullptr;
@@ -1885,8 +1893,10 @@ int egs_mloe_mmom_host(int n_obs, int n_miss, int dts, const double* x_obs, cons
     set_last_error("theta outside the Matern domain (sigma2 > 0, beta > 0, nu > 0)", "egs_mloe_mmom_host");
     return EGS_ERR_INVALID;
   }
-  // K_t, K_a: the observed covariance under the true / the estimated theta, factored
-  // pa is created first so that pt, which borrows pa's stream below, is destroyed first
+  // K_t, K_a: the observed covariance under the true / the estimated theta.  The
+  // two factorisations and forward solves are independent and latency-bound, so
+  // each problem keeps its own stream for them.
+  // pa is created first so that pt, whose stream pa's work waits on, is destroyed first
   egs_problem *pt = nullptr, *pa = nullptr;
   int rc = egs_problem_create(&pa, n_obs, dts);
   if (rc != EGS_OK) return rc;
@@ -1895,64 +1905,78 @@ int egs_mloe_mmom_host(int n_obs, int n_miss, int dts, const double* x_obs, cons
   std::unique_ptr<egs_problem, int (*)(egs_problem*)> gt(pt, egs_problem_destroy);
   for (egs_problem* p : {pt, pa}) {
     if ((rc = egs_problem_set_locations(p, x_obs, y_obs)) != EGS_OK) return rc;
-    p->have_observations = true;  // the solves below set z themselves
+    if ((rc = set_params(p, p == pt ? theta_true : theta_est)) != EGS_OK) return rc;
+    EGS_CUDA_TRY(cudaMemsetAsync(p->flags, 0, 2 * sizeof(int), p->stream));
+    if ((rc = launch_matern_tiles(p->tiles, p->x, p->y, p->n, p->ts, p->nt, p->dparams, p->ktab, p->stream)) != EGS_OK)
+      return rc;
+    if ((rc = enqueue_potrf(p)) != EGS_OK) return rc;
   }
-  if ((rc = egs_covariance_generate(pt, theta_true)) != EGS_OK || (rc = egs_potrf(pt)) != EGS_OK) return rc;
-  if ((rc = egs_covariance_generate(pa, theta_est)) != EGS_OK || (rc = egs_potrf(pa)) != EGS_OK) return rc;
-  // both problems run on pa's stream from here
-  cudaStream_t st = pa->stream;
-  const long long np = pa->np;
-  double *kt = nullptr, *ka = nullptr, *dxm = nullptr, *dym = nullptr, *ya = nullptr, *u = nullptr, *dots = nullptr;
+  if ((rc = sync_flags(pt, false)) != EGS_OK || (rc = sync_flags(pa, false)) != EGS_OK) return rc;
+  cudaStream_t st = pa->stream, st2 = pt->stream;
+  const int ts = pa->ts, nt = pa->nt, np = pa->np;
+  // targets in groups of at most 512, as the rows of a matrix (64-row chunks)
+  const int group = std::min((n_miss + kInnerBlock - 1) / kInnerBlock * kInnerBlock, 512);
+  double *ya = nullptr, *xa = nullptr, *yt = nullptr, *xt = nullptr, *dxm = nullptr, *dym = nullptr, *dots = nullptr;
   long long dummy = 0;
+  cudaEvent_t ready = nullptr;
   auto cleanup = [&]() {
-    for (void* b : {(void*)kt, (void*)ka, (void*)dxm, (void*)dym, (void*)ya, (void*)u, (void*)dots}) dev_free(b, st);
+    cudaStreamSynchronize(st2);
+    for (void* b : {(void*)ya, (void*)xa, (void*)yt, (void*)xt, (void*)dxm, (void*)dym, (void*)dots}) dev_free(b, st);
     cudaStreamSynchronize(st);
+    if (ready) cudaEventDestroy(ready);
   };
-  if ((rc = dev_alloc(&kt, (size_t)np * n_miss, &dummy, st)) || (rc = dev_alloc(&ka, (size_t)np * n_miss, &dummy, st)) ||
+  const size_t block = (size_t)group * np;
+  if ((rc = dev_alloc(&ya, 2 * block, &dummy, st)) || (rc = dev_alloc(&xa, 2 * block, &dummy, st)) ||
+      (rc = dev_alloc(&yt, block, &dummy, st)) || (rc = dev_alloc(&xt, block, &dummy, st)) ||
       (rc = dev_alloc(&dxm, n_miss, &dummy, st)) || (rc = dev_alloc(&dym, n_miss, &dummy, st)) ||
-      (rc = dev_alloc(&ya, np, &dummy, st)) || (rc = dev_alloc(&u, np, &dummy, st)) ||
       (rc = dev_alloc(&dots, (size_t)4 * n_miss, &dummy, st))) {
     cleanup();
     return rc;
   }
-  cudaMemsetAsync(kt, 0, (size_t)np * n_miss * sizeof(double), st);
-  cudaMemsetAsync(ka, 0, (size_t)np * n_miss * sizeof(double), st);
+  if (cudaEventCreateWithFlags(&ready, cudaEventDisableTiming) != cudaSuccess) {
+    cudaGetLastError();
+    set_last_error("event creation failed", "egs_mloe_mmom_host");
+    cleanup();
+    return EGS_ERR_CUDA;
+  }
   cudaMemcpyAsync(dxm, x_miss, n_miss * sizeof(double), cudaMemcpyHostToDevice, st);
   cudaMemcpyAsync(dym, y_miss, n_miss * sizeof(double), cudaMemcpyHostToDevice, st);
-  // k_t, k_a for every target: columns of leading dimension np (padding rows stay 0)
-  if ((rc = launch_matern_block(kt, (int)np, n_obs, n_miss, pa->x, pa->y, dxm, dym, mt, st)) != EGS_OK ||
-      (rc = launch_matern_block(ka, (int)np, n_obs, n_miss, pa->x, pa->y, dxm, dym, ma, st)) != EGS_OK ||
-      (rc = egs_problem_set_stream(pt, st)) != EGS_OK) {
-    cleanup();
-    return rc;
-  }
-  for (int q = 0; q < n_miss; ++q) {
-    const double* ktq = kt + (long long)q * np;
-    const double* kaq = ka + (long long)q * np;
-    double* d = dots + 4ll * q;
-    // y_a = L_a^-1 k_a
-    cudaMemcpyAsync(pa->z, kaq, np * sizeof(double), cudaMemcpyDeviceToDevice, st);
-    enqueue_trsv(pa);
-    cudaMemcpyAsync(ya, pa->z, np * sizeof(double), cudaMemcpyDeviceToDevice, st);
-    launch_dot(ya, ya, (int)np, d + 0, st);                       // k_a' K_a^-1 k_a
-    // L_a^-1 k_t . y_a = k_t' K_a^-1 k_a
-    cudaMemcpyAsync(pa->z, ktq, np * sizeof(double), cudaMemcpyDeviceToDevice, st);
-    enqueue_trsv(pa);
-    launch_dot(pa->z, ya, (int)np, d + 1, st);
-    // k_t' K_t^-1 k_t
-    cudaMemcpyAsync(pt->z, ktq, np * sizeof(double), cudaMemcpyDeviceToDevice, st);
-    enqueue_trsv(pt);
-    launch_dot(pt->z, pt->z, (int)np, d + 2, st);
+  for (int q0 = 0; q0 < n_miss && rc == EGS_OK; q0 += group) {
+    const int m = std::min(group, n_miss - q0);
+    const long long lda = 2LL * group, ldt = group;  // ya, xa: k_a rows, then k_t rows
+    const double *xm = dxm + q0, *ym = dym + q0;
+    double* d = dots + 4LL * q0;
+    cudaMemsetAsync(ya, 0, 2 * block * sizeof(double), st);
+    cudaMemsetAsync(yt, 0, block * sizeof(double), st);
+    // k_a and k_t of every target (padding rows and columns stay 0)
+    if ((rc = launch_matern_block(ya, (int)lda, m, n_obs, xm, ym, pa->x, pa->y, ma, st)) != EGS_OK ||
+        (rc = launch_matern_block(ya + group, (int)lda, m, n_obs, xm, ym, pa->x, pa->y, mt, st)) != EGS_OK)
+      break;
+    cudaMemcpy2DAsync(yt, ldt * sizeof(double), ya + group, lda * sizeof(double), ldt * sizeof(double), np,
+                      cudaMemcpyDeviceToDevice, st);
+    cudaEventRecord(ready, st);
+    cudaStreamWaitEvent(st2, ready, 0);
+    // L_t^-1 k_t beside L_a^-1 [k_a, k_t] = [y_a, y_t]
+    if ((rc = launch_rows_forward(pt->tiles, ts, nt, yt, xt, ldt, group, st2)) != EGS_OK ||
+        (rc = launch_rows_forward(pa->tiles, ts, nt, ya, xa, lda, 2 * group, st)) != EGS_OK)
+      break;
+    cudaEventRecord(ready, st2);
+    launch_rows_dot(xa, xa, lda, np, m, d + 0, 4, st);          // k_a' K_a^-1 k_a
+    launch_rows_dot(xa + group, xa, lda, np, m, d + 1, 4, st);  // k_t' K_a^-1 k_a
     // w_a = L_a^-T y_a; w_a' K_t w_a = |L_t^T w_a|^2
-    cudaMemcpyAsync(pa->z, ya, np * sizeof(double), cudaMemcpyDeviceToDevice, st);
-    enqueue_trsv_t(pa);
-    launch_trmv_t(pt->tiles, pt->ts, pt->nt, pa->z, u, st);
-    launch_dot(u, u, (int)np, d + 3, st);
+    if ((rc = launch_rows_backward(pa->tiles, ts, nt, xa, ya, lda, group, st)) != EGS_OK) break;
+    cudaStreamWaitEvent(st, ready, 0);
+    launch_rows_dot(xt, xt, ldt, np, m, d + 2, 4, st);          // k_t' K_t^-1 k_t
+    if ((rc = launch_rows_times_lower(pt->tiles, ts, nt, ya, ya + group, lda, group, st)) != EGS_OK) break;
+    launch_rows_dot(ya + group, ya + group, lda, np, m, d + 3, 4, st);
+    rc = check_cuda("egs_mloe_mmom_host");
   }
   std::vector<double> h(4ll * n_miss);
-  cudaMemcpyAsync(h.data(), dots, h.size() * sizeof(double), cudaMemcpyDeviceToHost, st);
-  rc = check_cuda("egs_mloe_mmom_host");
-  if (cudaStreamSynchronize(st) != cudaSuccess && rc == EGS_OK) rc = check_cuda("egs_mloe_mmom_host/sync");
+  if (rc == EGS_OK) {
+    cudaMemcpyAsync(h.data(), dots, h.size() * sizeof(double), cudaMemcpyDeviceToHost, st);
+    rc = check_cuda("egs_mloe_mmom_host");
+    if (cudaStreamSynchronize(st) != cudaSuccess && rc == EGS_OK) rc = check_cuda("egs_mloe_mmom_host/sync");
+  }
   cleanup();
   if (rc != EGS_OK) return rc;
   const double s2t = theta_true[0], s2a = theta_est[0];

@@ -41,10 +41,20 @@ int panel_outer_blocks(int ts, int kb);
 int launch_panel_step(double* col, int ts, int rows_below, int kb, int nb, int gcol, int* info, double* z,
                       PanelChain& ch, cudaStream_t st);
 int launch_panel_flush(PanelChain& ch, cudaStream_t st);
-void launch_trsv_diag(const double* tiles, int ts, long long slot, double* zk, cudaStream_t st);
-void launch_gemv_panel(const double* tiles, int ts, int nt, int k, double* z, cudaStream_t st);
-void launch_trsv_t_diag(const double* tiles, int ts, long long slot, double* zk, cudaStream_t st);
-void launch_gemv_t_panel(const double* tiles, int ts, int nt, int k, double* z, cudaStream_t st);
+// Triangular solves against a finished factor (solve.cu): one vector in place
+// (scratch: 128 doubles), or the rows of a matrix.
+int launch_vec_forward(const double* tiles, int ts, int nt, double* z, double* scratch, cudaStream_t st,
+                       long long* launches);
+int launch_vec_backward(const double* tiles, int ts, int nt, double* z, double* scratch, cudaStream_t st,
+                        long long* launches);
+int launch_rows_forward(const double* tiles, int ts, int nt, double* Y, double* X, long long ldy, int rows,
+                        cudaStream_t st);
+int launch_rows_backward(const double* tiles, int ts, int nt, double* Y, double* X, long long ldy, int rows,
+                         cudaStream_t st);
+int launch_rows_times_lower(const double* tiles, int ts, int nt, const double* W, double* U, long long ldy, int rows,
+                            cudaStream_t st);
+void launch_rows_dot(const double* A, const double* B, long long ldy, int np, int m, double* out, int stride,
+                     cudaStream_t st);
 void launch_logdet_partials(const double* tiles, int ts, int nt, int n, double* partial, cudaStream_t st);
 void launch_finalize(const double* partial, int nt, const double* z, int n, double* result,
                      const int* info, cudaStream_t st);
@@ -117,8 +127,6 @@ void launch_scatter_panel(const double* W2, double* band, double* inv, double* W
                           cudaStream_t st);
 void launch_scatter_offband(const double* W, float* off, int ts, int nt, int b, int nb, int k, cudaStream_t st);
 const float* offband_tile(const float* off, int ts, int nt, int b, int i, int k);
-void launch_trmv_t(const double* tiles, int ts, int nt, const double* w, double* out, cudaStream_t st);
-void launch_dot(const double* a, const double* b, int n, double* out, cudaStream_t st);
 long long residual_scratch_doubles(int n);
 void launch_add_inplace(double* a, const double* b, int n, cudaStream_t st);
 void launch_matern_residual(const double* x, const double* y, const double* z, const double* v, int n, int np,

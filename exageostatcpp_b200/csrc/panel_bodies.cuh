@@ -21,54 +21,6 @@ __device__ __forceinline__ double block_sum_256(double v, double* red) {
   return out;
 }
 
-// Forward substitution on one diagonal tile T: zk := T^-1 zk (ts entries).
-// Dynamic shared memory: ts doubles.
-__device__ __forceinline__ void trsv_diag_body(const double* __restrict__ T, int ts, double* __restrict__ zk) {
-  extern __shared__ double zs[];  // ts
-  __shared__ double B[kNB][kNB + 1];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int r = tid; r < ts; r += blockDim.x) zs[r] = zk[r];
-  for (int kb = 0; kb < ts; kb += kNB) {
-    for (int e = tid; e < kNB * kNB; e += blockDim.x) {
-      const int rr = e % kNB, c = e / kNB;
-      B[rr][c] = (rr >= c) ? T[(long long)(kb + c) * ts + kb + rr] : 0.0;
-    }
-    __syncthreads();
-    if (warp == 0) {
-      double z0 = zs[kb + lane], z1 = zs[kb + 32 + lane];
-      for (int c = 0; c < kNB; ++c) {
-        double zc;
-        if (c < 32) {
-          if (lane == c) z0 = z0 / B[c][c];
-          zc = __shfl_sync(0xffffffffu, z0, c);
-        } else {
-          if (lane == c - 32) z1 = z1 / B[c][c];
-          zc = __shfl_sync(0xffffffffu, z1, c - 32);
-        }
-        if (lane > c) z0 = fma(-B[lane][c], zc, z0);
-        if (lane + 32 > c) z1 = fma(-B[lane + 32][c], zc, z1);
-      }
-      zs[kb + lane] = z0;
-      zs[kb + 32 + lane] = z1;
-    }
-    __syncthreads();
-    for (int r = kb + kNB + tid; r < ts; r += blockDim.x) {
-      const double* col = T + (long long)kb * ts + r;
-      double acc0 = 0.0, acc1 = 0.0, acc2 = 0.0, acc3 = 0.0;
-#pragma unroll 4
-      for (int c = 0; c < kNB; c += 4) {
-        acc0 = fma(col[(long long)c * ts], zs[kb + c], acc0);
-        acc1 = fma(col[(long long)(c + 1) * ts], zs[kb + c + 1], acc1);
-        acc2 = fma(col[(long long)(c + 2) * ts], zs[kb + c + 2], acc2);
-        acc3 = fma(col[(long long)(c + 3) * ts], zs[kb + c + 3], acc3);
-      }
-      zs[r] -= (acc0 + acc1) + (acc2 + acc3);
-    }
-    __syncthreads();
-  }
-  for (int r = tid; r < ts; r += blockDim.x) zk[r] = zs[r];
-}
-
 // zi -= T zk for the 64 rows of block rblk of tile T (256 threads = 64 rows x
 // 4 column groups, fixed reduction order, FP64 arithmetic whatever the tile's
 // storage type).  Dynamic shared memory: ts doubles.

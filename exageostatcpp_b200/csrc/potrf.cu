@@ -1,7 +1,6 @@
 // Panel-level building blocks of the tiled Cholesky path on sm_100a: the 64-column
-// panel step (diagonal block, row solve and update in one launch), the single
-// right-hand-side forward/backward substitution over tiles,
-// and the deterministic reductions that turn the factor into the log-likelihood.
+// panel step (diagonal block, row solve and update in one launch) and the
+// deterministic reductions that turn the factor into the log-likelihood.
 //
 // Reference counterparts:
 //   CHAMELEON_dpotrf_Tile            ChameleonDense.cpp:25-37   (panel part; the trailing
@@ -86,103 +85,6 @@ int launch_panel_flush(PanelChain& ch, cudaStream_t st) {
   panel_flush_kernel<<<ch.chunks, kStepThreads, 0, st>>>(slot, ch.col, ch.ts, ch.kb, ch.z);
   ch.chunks = 0;
   return launch_status("panel_flush_kernel");
-}
-
-// Forward substitution on one diagonal tile: z_k := L_kk^-1 z_k (trsv_diag_body).
-__global__ void __launch_bounds__(1024)
-trsv_diag_kernel(const double* __restrict__ tiles, int ts, long long slot, double* __restrict__ zk) {
-  trsv_diag_body(tiles + slot * (long long)ts * ts, ts, zk);
-}
-
-void launch_trsv_diag(const double* tiles, int ts, long long slot, double* zk, cudaStream_t st) {
-  trsv_diag_kernel<<<1, 1024, ts * sizeof(double), st>>>(tiles, ts, slot, zk);
-}
-
-// z_i -= L_ik z_k for every tile row i > k (gemv_panel_body).
-__global__ void __launch_bounds__(256)
-gemv_panel_kernel(const double* __restrict__ tiles, int ts, int nt, int k, double* __restrict__ z) {
-  const int i = k + 1 + blockIdx.y;
-  gemv_panel_body(tiles + tile_slot(i, k, nt) * (long long)ts * ts, ts, z + (long long)k * ts,
-                  z + (long long)i * ts, blockIdx.x);
-}
-
-void launch_gemv_panel(const double* tiles, int ts, int nt, int k, double* z, cudaStream_t st) {
-  if (k >= nt - 1) return;
-  gemv_panel_kernel<<<dim3((ts + kNB - 1) / kNB, nt - 1 - k), 256, ts * sizeof(double), st>>>(tiles, ts, nt,
-                                                                                          k, z);
-}
-
-// ---------------------------------------------------------------------------
-// Backward substitution on one diagonal tile: z_k := L_kk^-T z_k.
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256)
-trsv_t_diag_kernel(const double* __restrict__ tiles, int ts, long long slot, double* __restrict__ zk) {
-  extern __shared__ double zs[];
-  __shared__ double B[kNB][kNB + 1];
-  const double* T = tiles + slot * (long long)ts * ts;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int r = tid; r < ts; r += blockDim.x) zs[r] = zk[r];
-  for (int kb = ts - kNB; kb >= 0; kb -= kNB) {
-    for (int e = tid; e < kNB * kNB; e += blockDim.x) {
-      const int rr = e % kNB, c = e / kNB;
-      B[rr][c] = (rr >= c) ? T[(long long)(kb + c) * ts + kb + rr] : 0.0;
-    }
-    __syncthreads();
-    if (warp == 0) {
-      double z0 = zs[kb + lane], z1 = zs[kb + 32 + lane];
-      for (int c = kNB - 1; c >= 0; --c) {
-        double zc;
-        if (c >= 32) {
-          if (lane == c - 32) z1 = z1 / B[c][c];
-          zc = __shfl_sync(0xffffffffu, z1, c - 32);
-        } else {
-          if (lane == c) z0 = z0 / B[c][c];
-          zc = __shfl_sync(0xffffffffu, z0, c);
-        }
-        // rows r < c: z_r -= L[c][r] x_c
-        if (lane < c) z0 = fma(-B[c][lane], zc, z0);
-        if (lane + 32 < c) z1 = fma(-B[c][lane + 32], zc, z1);
-      }
-      zs[kb + lane] = z0;
-      zs[kb + 32 + lane] = z1;
-    }
-    __syncthreads();
-    // rows r < kb: z_r -= sum_c L[kb+c][r] x[kb+c]; column r of L is contiguous in rows.
-    for (int r = warp; r < kb; r += blockDim.x / 32) {
-      const double* col = T + (long long)r * ts + kb;
-      double acc = fma(col[lane], zs[kb + lane], col[lane + 32] * zs[kb + lane + 32]);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-      if (lane == 0) zs[r] -= acc;
-    }
-    __syncthreads();
-  }
-  for (int r = tid; r < ts; r += blockDim.x) zk[r] = zs[r];
-}
-
-void launch_trsv_t_diag(const double* tiles, int ts, long long slot, double* zk, cudaStream_t st) {
-  trsv_t_diag_kernel<<<1, 256, ts * sizeof(double), st>>>(tiles, ts, slot, zk);
-}
-
-// z_i -= L_ki^T z_k for every tile column i < k (tile (k, i) is stored).  One warp per column.
-__global__ void __launch_bounds__(256)
-gemv_t_panel_kernel(const double* __restrict__ tiles, int ts, int nt, int k, double* __restrict__ z) {
-  const int i = blockIdx.y;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int c = blockIdx.x * 8 + warp;
-  if (c >= ts) return;
-  const double* col = tiles + tile_slot(k, i, nt) * (long long)ts * ts + (long long)c * ts;
-  const double* zk = z + (long long)k * ts;
-  double acc = 0.0;
-  for (int r = lane; r < ts; r += 32) acc = fma(col[r], zk[r], acc);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if (lane == 0) z[(long long)i * ts + c] -= acc;
-}
-
-void launch_gemv_t_panel(const double* tiles, int ts, int nt, int k, double* z, cudaStream_t st) {
-  if (k <= 0) return;
-  gemv_t_panel_kernel<<<dim3((ts + 7) / 8, k), 256, 0, st>>>(tiles, ts, nt, k, z);
 }
 
 // ---------------------------------------------------------------------------
@@ -303,48 +205,6 @@ void launch_trmv(const double* tiles, int ts, int nt, const double* e, double* p
   trmv_tile_kernel<<<dim3((ts + kNB - 1) / kNB, (unsigned)nslots), 256, 0, st>>>(tiles, ts, nt, e, part);
   const long long total = (long long)nt * ts;
   trmv_reduce_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(part, ts, nt, z);
-}
-
-}  // namespace egs
-
-namespace egs {
-
-// out = L^T w for the lower tiled factor (global row r = j ts + c):
-// out[r] = sum_{i > j} (column c of tile (i, j)) . w_i + sum_{rr >= c} L_jj(rr, c) w_j(rr);
-// one warp per output element, fixed summation order.
-__global__ void __launch_bounds__(256)
-trmv_t_kernel(const double* __restrict__ tiles, int ts, int nt, const double* __restrict__ w,
-              double* __restrict__ out) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int j = blockIdx.y, c = blockIdx.x * 8 + warp;
-  if (c >= ts) return;
-  double acc = 0.0;
-  for (int i = j; i < nt; ++i) {
-    const double* col = tiles + tile_slot(i, j, nt) * (long long)ts * ts + (long long)c * ts;
-    const double* wi = w + (long long)i * ts;
-    for (int rr = (i == j ? c : 0) + lane; rr < ts; rr += 32) acc = fma(col[rr], wi[rr], acc);
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if (lane == 0) out[(long long)j * ts + c] = acc;
-}
-
-void launch_trmv_t(const double* tiles, int ts, int nt, const double* w, double* out, cudaStream_t st) {
-  trmv_t_kernel<<<dim3((ts + 7) / 8, nt), 256, 0, st>>>(tiles, ts, nt, w, out);
-}
-
-// out[slot] = a . b over n entries (one block, fixed order).
-__global__ void __launch_bounds__(256)
-dot_kernel(const double* __restrict__ a, const double* __restrict__ b, int n, double* __restrict__ out) {
-  __shared__ double red[256];
-  double acc = 0.0;
-  for (int i = threadIdx.x; i < n; i += 256) acc = fma(a[i], b[i], acc);
-  const double s = block_sum_256(acc, red);
-  if (threadIdx.x == 0) *out = s;
-}
-
-void launch_dot(const double* a, const double* b, int n, double* out, cudaStream_t st) {
-  dot_kernel<<<1, 256, 0, st>>>(a, b, n, out);
 }
 
 }  // namespace egs
