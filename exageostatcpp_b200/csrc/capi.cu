@@ -359,21 +359,20 @@ int enqueue_panel(double* tiles, const void* tmap, int ts, int nt, int row_tiles
 // Step k: the panel of tile column k (enqueue_panel), then the tensor-core
 // trailing update of every tile (i, j), k < j <= i.  z (or null) is a vector of
 // np entries that becomes L^-1 z with the panels.
-int enqueue_potrf(egs_problem* p, double* z = nullptr, int steps = -1) {
+int enqueue_potrf(egs_problem* p, double* z = nullptr) {
   const int ts = p->ts, nt = p->nt, n = p->n;
   cudaStream_t st = p->stream;
   int* info = p->flags;
   int* err = p->flags + 1;
-  const int kend = (steps >= 0 && steps < nt) ? steps : nt;
   PanelChain ch;
   ch.scratch = p->pscratch;
-  for (int k = 0; k < kend; ++k) {
+  for (int k = 0; k < nt; ++k) {
     int sp = span_begin(p, EGS_STAGE_PANEL);
     long long nl = 0;
     int rc = enqueue_panel(p->tiles, p->tmap, ts, nt, nt, k, k * ts, info, err,
                            z ? z + (long long)k * ts : nullptr, ch, st, &nl);
     if (rc != EGS_OK) return rc;
-    if (k == kend - 1) {
+    if (k == nt - 1) {
       if ((rc = launch_panel_flush(ch, st)) != EGS_OK) return rc;
       ++nl;
     }
@@ -1907,9 +1906,8 @@ int egs_mloe_mmom_host(int n_obs, int n_miss, int dts, const double* x_obs, cons
     if ((rc = egs_problem_set_locations(p, x_obs, y_obs)) != EGS_OK) return rc;
     if ((rc = set_params(p, p == pt ? theta_true : theta_est)) != EGS_OK) return rc;
     EGS_CUDA_TRY(cudaMemsetAsync(p->flags, 0, 2 * sizeof(int), p->stream));
-    if ((rc = launch_matern_tiles(p->tiles, p->x, p->y, p->n, p->ts, p->nt, p->dparams, p->ktab, p->stream)) != EGS_OK)
-      return rc;
-    if ((rc = enqueue_potrf(p)) != EGS_OK) return rc;
+    rc = launch_matern_tiles(p->tiles, p->x, p->y, p->n, p->ts, p->nt, p->dparams, p->ktab, p->stream);
+    if (rc != EGS_OK || (rc = enqueue_potrf(p)) != EGS_OK) return rc;
   }
   if ((rc = sync_flags(pt, false)) != EGS_OK || (rc = sync_flags(pa, false)) != EGS_OK) return rc;
   cudaStream_t st = pa->stream, st2 = pt->stream;
@@ -2001,29 +1999,21 @@ int egs_mloe_mmom_host(int n_obs, int n_miss, int dts, const double* x_obs, cons
 
 namespace egs {
 
-// The first `steps` tile steps of the factorisation of p's tiles as they are
-// (no generation): the panels of columns 0 .. steps-1 and their trailing
-// updates of every later tile.  Used by the Fisher information
-// (augmented matrices).  Returns the LAPACK-style info or an error.
-int enqueue_potrf_steps(egs_problem* p, int steps) {
-  EGS_CUDA_TRY(cudaMemsetAsync(p->flags, 0, 2 * sizeof(int), p->stream));
-  int rc = enqueue_potrf(p, nullptr, steps);
+// C(theta) generated and factored in p's tiles (used by the Fisher information).
+// Returns the LAPACK-style info or an error.
+int factor_resident(egs_problem* p, const double* theta) {
+  int rc = set_params(p, theta);
   if (rc != EGS_OK) return rc;
-  EGS_CUDA_TRY(cudaMemcpyAsync(p->hflags, p->flags, 2 * sizeof(int), cudaMemcpyDeviceToHost, p->stream));
-  EGS_CUDA_TRY(cudaStreamSynchronize(p->stream));
-  if (p->hflags[1] != 0) {
-    set_last_error("a device-side wait exceeded its limit", "enqueue_potrf_steps");
-    return EGS_ERR_TIMEOUT;
-  }
-  if (p->hflags[0] > 0) {
-    set_last_error("Matrix is not positive definite", "enqueue_potrf_steps");
-    return p->hflags[0];
-  }
-  return check_cuda("enqueue_potrf_steps");
+  EGS_CUDA_TRY(cudaMemsetAsync(p->flags, 0, 2 * sizeof(int), p->stream));
+  rc = launch_matern_tiles(p->tiles, p->x, p->y, p->n, p->ts, p->nt, p->dparams, p->ktab, p->stream);
+  if (rc != EGS_OK || (rc = enqueue_potrf(p)) != EGS_OK) return rc;
+  return sync_flags(p, false);
 }
 
-int problem_tiles(egs_problem* p, double** tiles, int* ts, int* nt, cudaStream_t* st) {
+int problem_tiles(egs_problem* p, double** tiles, double** x, double** y, int* ts, int* nt, cudaStream_t* st) {
   *tiles = p->tiles;
+  *x = p->x;
+  *y = p->y;
   *ts = p->ts;
   *nt = p->nt;
   *st = p->stream;

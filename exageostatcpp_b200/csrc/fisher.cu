@@ -6,11 +6,9 @@
 // with two triangular solves per derivative and one dense product plus a
 // trace per pair, and returns A^-1.  Here the same quantity is computed as
 //     A_jk = 1/2 sum(M_j o M_k),   M_j = L^-1 C_j L^-T  (symmetric),
-// which needs no N^3 product per pair.  M_j comes from two partial tiled
-// Cholesky factorisations of the augmented matrix [[C, .], [B, I]]: the first
-// nt tile steps leave B L^-T in the lower-left block, so B = C_j gives
-// Y = C_j L^-T and then B = Y^T = L^-1 C_j gives L^-1 C_j L^-T = M_j.  Everything runs on
-// the library's own tile kernels (64x64 potrf, row solves, DMMA updates).
+// which needs no N^3 product per pair.  C is factored once; the rows of the three
+// symmetric C_j, stacked, go through two row solves: X_j = C_j L^-T, then X_j^T L^-T =
+// L^-1 C_j L^-T = M_j (solve.cu).
 //
 // Derivative kernels (src/kernels/concrete/UnivariateMaternDdsigmaSquare.cpp,
 // UnivariateMaternDbeta.cpp, UnivariateMaternDnu.cpp): at scaled distance
@@ -20,10 +18,12 @@
 //     dC/dnu     = sigma2 [-2 ln2 2^-nu / Gamma(nu) x^nu K_nu + 2^(1-nu) (-psi(nu)/Gamma(nu) x^nu K_nu
 //                          + (x^nu ln x K_nu + x^nu dK_nu/dnu) / Gamma(nu))]  (0 at x = 0).
 // The reference differentiates K_nu in nu by a forward difference with step
-// 1e-9 (src/helpers/BasselFunction.cpp:23-33); here central differences at
-// steps 1e-3 and 5e-4 over the library's K_nu (Temme series / Steed CF2,
-// ~1e-13 relative), combined by Richardson extrapolation, give dK/dnu to
-// ~1e-9, well inside the reference's own noise.
+// 1e-9 (src/helpers/BasselFunction.cpp:23-33); here F_nu(x) = x^nu K_nu(x) itself is
+// differentiated: the last two terms are dF/dnu, from the six-point central
+// difference with step h = 2e-3 (truncation h^6 / 140 d^7F/dnu^7), and dC/dbeta = sigma2 c (F_nu+1 - 2 nu F_nu) / beta.  F comes from the Chebyshev
+// tables of the generator (e^x F, one table per nu value), where the direct
+// series and continued fraction cost thousands of operations for every order
+// (N = 1,600: derivatives 2.7 ms of direct evaluations, 0.1 from the tables).
 #include <cmath>
 #include <memory>
 #include <vector>
@@ -32,149 +32,119 @@
 
 namespace egs {
 
-// K_nu(x) and K_{nu+1}(x) for any nu >= 0, x > 0 (unscaled).
-__device__ __forceinline__ void bessel_k_pair(double nu, double x, double& knu, double& knu1) {
-  const int n = (int)floor(nu + 0.5);
-  const double mu = nu - n;
-  double k0, k1;
-  bool scaled;
-  if (x <= 2.0) {
-    k_temme_series(mu, x, k0, k1);
-    scaled = false;
-  } else {
-    k_steed_cf2_scaled(mu, x, k0, k1);
-    scaled = true;
-  }
-  double v = mu + 1.0;
-  for (int j = 0; j < n; ++j) {  // (K_mu+j, K_mu+j+1) -> (K_mu+j+1, K_mu+j+2)
-    const double k2 = k0 + (2.0 * v / x) * k1;
-    k0 = k1;
-    k1 = k2;
-    v += 1.0;
-  }
-  if (scaled) {
-    const double e = exp(-x);
-    k0 *= e;
-    k1 *= e;
-  }
-  knu = k0;
-  knu1 = k1;
-}
-
 struct FisherParams {
   double sigma2, beta, nu;
   double con;    // 1 / (2^(nu-1) Gamma(nu))
-  double ginv;   // 1 / Gamma(nu)
   double psi;    // digamma(nu)
 };
 
-// The three derivative matrices, dense column-major np x np (rows / columns
-// past n are zero): d[j * np * np + c * np + r].
+// Orders whose F the derivatives need: nu, nu + 1, nu +- h, nu +- 2 h, nu +- 3 h.
+constexpr int kFisherOrders = 8;
+constexpr double kFisherStep = 2e-3;
+constexpr int kFisherTabBytes = kFisherOrders * kKtabDoubles * (int)sizeof(double);
+
+// F_nu(x) = x^nu K_nu(x) of the order of p (kind 2), from its table where x lies in it.
+__device__ __forceinline__ double bessel_f(double x, bool in_table, int idx, double t, double ex,
+                                           const MaternParams& p, const double* __restrict__ tab) {
+  if (in_table && p.table) return ktab_sum(tab + idx * kKtabStride, t) * ex;
+  bool scaled;
+  const double k = bessel_k_general(x, p, scaled);
+  return pow(x, p.nu) * (scaled ? k * ex : k);
+}
+
+// The three derivative matrices stacked as rows, column-major with column stride
+// 3 np (rows / columns past n are zero): d[c * 3 np + j * np + r].
 __global__ void __launch_bounds__(256)
 matern_derivatives_kernel(const double* __restrict__ x, const double* __restrict__ y, int n, int np,
-                          FisherParams q, double* __restrict__ d) {
-  const long long idx = (long long)blockIdx.x * 256 + threadIdx.x;
-  const long long nn = (long long)np * np;
-  if (idx >= nn) return;
-  const int c = (int)(idx / np), r = (int)(idx - (long long)c * np);
-  double ds = 0.0, db = 0.0, dn = 0.0;
-  if (r < n && c < n) {
-    const double e = euclid_dist(x[r], y[r], x[c], y[c]) / q.beta;
-    if (e == 0.0) {
-      ds = 1.0;
-    } else {
-      double k0, k1, kp, km, kq, kr, unused;
-      bessel_k_pair(q.nu, e, k0, k1);
-      // central differences at h and h/2 combined by Richardson extrapolation:
-      // O(h^4) truncation, ~1e-13 / h rounding
-      const double h = 1e-3;
-      bessel_k_pair(q.nu + h, e, kp, unused);
-      bessel_k_pair(q.nu - h, e, km, unused);
-      bessel_k_pair(q.nu + 0.5 * h, e, kq, unused);
-      bessel_k_pair(q.nu - 0.5 * h, e, kr, unused);
-      const double d1 = (kp - km) / (2.0 * h), d2 = (kq - kr) / h;
-      const double dk = (4.0 * d2 - d1) / 3.0;
-      const double xn = pow(e, q.nu);
-      ds = q.con * xn * k0;
-      db = q.sigma2 * q.con * (-q.nu / q.beta * xn * k0 - xn * (q.nu / e * k0 - k1) * e / q.beta);
-      dn = q.sigma2 * (-2.0 * log(2.0) * pow(2.0, -q.nu) * q.ginv * xn * k0 +
-                       pow(2.0, 1.0 - q.nu) * (-q.psi * q.ginv * xn * k0 + (xn * log(e) * k0 + xn * dk) * q.ginv));
-    }
-  }
-  d[idx] = ds;
-  d[nn + idx] = db;
-  d[2 * nn + idx] = dn;
-}
-
-// Lower tiles of the augmented 2nt x 2nt matrix [[C, .], [B, I]] from dense
-// np x np column-major C (lower part used) and B.
-// transB: take B transposed (B^T(r, c) = B[r * np + c]).
-__global__ void __launch_bounds__(256)
-augment_tiles_kernel(double* __restrict__ tiles, int ts, int nt, const double* __restrict__ C,
-                     const double* __restrict__ B, int transB) {
-  const int nt2 = 2 * nt;
-  const long long slot = blockIdx.y;
-  // slot -> (i, j) of the lower layout of nt2 tiles
-  int j = 0;
-  long long s = slot;
-  while (s >= nt2 - j) {
-    s -= nt2 - j;
-    ++j;
-  }
-  const int i = j + (int)s;
-  const long long np = (long long)nt * ts;
-  double* t = tiles + slot * (long long)ts * ts;
-  for (long long e = (long long)blockIdx.x * 256 + threadIdx.x; e < (long long)ts * ts; e += (long long)gridDim.x * 256) {
-    const int c = (int)(e / ts), r = (int)(e - (long long)c * ts);
-    double v;
-    if (i < nt) {
-      v = C[(long long)(j * ts + c) * np + i * ts + r];
-    } else if (j < nt) {
-      const long long br = (long long)(i - nt) * ts + r, bc = (long long)j * ts + c;
-      v = transB ? B[br * np + bc] : B[bc * np + br];
-    } else {
-      v = (i == j && r == c) ? 1.0 : 0.0;
-    }
-    t[e] = v;
-  }
-}
-
-// Dense np x np Y from the lower-left block tiles (nt + i, j).
-__global__ void __launch_bounds__(256)
-extract_block_kernel(const double* __restrict__ tiles, int ts, int nt, double* __restrict__ Y) {
-  const long long np = (long long)nt * ts;
-  const long long idx = (long long)blockIdx.x * 256 + threadIdx.x;
-  if (idx >= np * np) return;
-  const int c = (int)(idx / np), r = (int)(idx - (long long)c * np);
-  const int i = r / ts, j = c / ts;
-  const long long slot = tile_slot(nt + i, j, 2 * nt);
-  Y[idx] = tiles[slot * (long long)ts * ts + (long long)(c - j * ts) * ts + (r - i * ts)];
-}
-
-// Deterministic dot product of long vectors: per-block partial sums in a fixed
-// order, then one block adds the partials in order.
-__global__ void __launch_bounds__(256)
-dot_partial_kernel(const double* __restrict__ a, const double* __restrict__ b, long long n,
-                   double* __restrict__ partial) {
-  __shared__ double red[256];
-  double acc = 0.0;
-  for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n; i += (long long)gridDim.x * 256)
-    acc = fma(a[i], b[i], acc);
-  red[threadIdx.x] = acc;
+                          FisherParams q, const MaternParams* __restrict__ orders, const double* __restrict__ tabs,
+                          double* __restrict__ d) {
+  extern __shared__ double stab[];  // kFisherTabBytes
+  for (int i = threadIdx.x; i < kFisherOrders * kKtabDoubles; i += 256) stab[i] = tabs[i];
   __syncthreads();
-  for (int s = 128; s > 0; s >>= 1) {
-    if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
+  const long long nn = (long long)np * np;
+  for (long long idx = (long long)blockIdx.x * 256 + threadIdx.x; idx < nn; idx += (long long)gridDim.x * 256) {
+    const int c = (int)(idx / np), r = (int)(idx - (long long)c * np);
+    double ds = 0.0, db = 0.0, dn = 0.0;
+    if (r < n && c < n) {
+      const double e = euclid_dist(x[r], y[r], x[c], y[c]) / q.beta;
+      if (e == 0.0) {
+        ds = 1.0;
+      } else {
+        int at = 0;
+        double t = 0.0;
+        const bool in_table = ktab_locate(e, at, t);
+        const double ex = exp(-e);
+        double f[kFisherOrders];
+#pragma unroll
+        for (int o = 0; o < kFisherOrders; ++o)
+          f[o] = bessel_f(e, in_table, at, t, ex, orders[o], stab + o * kKtabDoubles);
+        const double df = (45.0 * (f[2] - f[3]) - 9.0 * (f[4] - f[5]) + (f[6] - f[7])) / (60.0 * kFisherStep);
+        ds = q.con * f[0];
+        db = q.sigma2 * q.con / q.beta * (f[1] - 2.0 * q.nu * f[0]);
+        dn = q.sigma2 * q.con * (df - (log(2.0) + q.psi) * f[0]);
+      }
+    }
+    double* out = d + (long long)c * 3 * np + r;
+    out[0] = ds;
+    out[np] = db;
+    out[2 * (long long)np] = dn;
+  }
+}
+
+// Y_j := X_j^T for the three stacked np x np matrices (64 x 64 blocks through
+// shared memory).
+__global__ void __launch_bounds__(256)
+transpose_stacked_kernel(const double* __restrict__ X, int np, double* __restrict__ Y) {
+  __shared__ double t[64][65];
+  const long long ld = 3LL * np;
+  const double* src = X + (long long)blockIdx.z * np;
+  double* dst = Y + (long long)blockIdx.z * np;
+  const int r0 = 64 * blockIdx.x, c0 = 64 * blockIdx.y, r = threadIdx.x & 63;
+  for (int c = threadIdx.x >> 6; c < 64; c += 4) t[c][r] = src[(c0 + c) * ld + r0 + r];
+  __syncthreads();
+  for (int c = threadIdx.x >> 6; c < 64; c += 4) dst[(r0 + c) * ld + c0 + r] = t[r][c];
+}
+
+// The six sums of M_j o M_k (j <= k) over the stacked matrices: per-block partial
+// sums in a fixed order, then one warp per pair adds the partials in a fixed order.
+constexpr int kPairs = 6;
+__global__ void __launch_bounds__(256)
+pair_dots_kernel(const double* __restrict__ M, int np, double* __restrict__ partial) {
+  __shared__ double red[256];
+  double acc[kPairs] = {};
+  const long long nn = (long long)np * np;
+  for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < nn; i += (long long)gridDim.x * 256) {
+    const long long c = i / np;
+    const double* m = M + c * 3 * np + (i - c * np);
+    const double a = m[0], b = m[np], d = m[2 * (long long)np];
+    acc[0] = fma(a, a, acc[0]);
+    acc[1] = fma(a, b, acc[1]);
+    acc[2] = fma(a, d, acc[2]);
+    acc[3] = fma(b, b, acc[3]);
+    acc[4] = fma(b, d, acc[4]);
+    acc[5] = fma(d, d, acc[5]);
+  }
+#pragma unroll
+  for (int q = 0; q < kPairs; ++q) {
+    red[threadIdx.x] = acc[q];
+    __syncthreads();
+    for (int s = 128; s > 0; s >>= 1) {
+      if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
+      __syncthreads();
+    }
+    if (threadIdx.x == 0) partial[blockIdx.x * kPairs + q] = red[0];
     __syncthreads();
   }
-  if (threadIdx.x == 0) partial[blockIdx.x] = red[0];
 }
 
-__global__ void sum_partials_kernel(const double* __restrict__ partial, int m, double* __restrict__ out) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    double s = 0.0;
-    for (int i = 0; i < m; ++i) s += partial[i];
-    *out = s;
-  }
+__global__ void __launch_bounds__(32 * kPairs)
+pair_sums_kernel(const double* __restrict__ partial, int m, double* __restrict__ out) {
+  const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double s = 0.0;
+  for (int i = lane; i < m; i += 32) s += partial[i * kPairs + q];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (lane == 0) out[q] = s;
 }
 
 }  // namespace egs
@@ -183,11 +153,12 @@ using namespace egs;
 
 namespace {
 
-// digamma(x), x > 0: recurrence psi(x) = psi(x+1) - 1/x up to x >= 6, then the
-// asymptotic series ln x - 1/(2x) - sum B_2k / (2k x^2k) (Abramowitz & Stegun 6.3.18).
+// digamma(x), x > 0: recurrence psi(x) = psi(x+1) - 1/x up to x >= 16, then the
+// asymptotic series ln x - 1/(2x) - sum B_2k / (2k x^2k) (Abramowitz & Stegun
+// 6.3.18), whose first omitted term is 0.021 / x^12 < 1e-16.
 double digamma(double x) {
   double r = 0.0;
-  while (x < 6.0) {
+  while (x < 16.0) {
     r -= 1.0 / x;
     x += 1.0;
   }
@@ -199,8 +170,8 @@ double digamma(double x) {
 }  // namespace
 
 namespace egs {
-int enqueue_potrf_steps(egs_problem* p, int steps);
-int problem_tiles(egs_problem* p, double** tiles, int* ts, int* nt, cudaStream_t* st);
+int factor_resident(egs_problem* p, const double* theta);
+int problem_tiles(egs_problem* p, double** tiles, double** x, double** y, int* ts, int* nt, cudaStream_t* st);
 }  // namespace egs
 
 extern "C" int egs_fisher_host(int n, int dts, const double* x, const double* y, const double* theta,
@@ -211,93 +182,80 @@ extern "C" int egs_fisher_host(int n, int dts, const double* x, const double* y,
     set_last_error("theta outside the Matern domain (sigma2 > 0, beta > 0, nu > 0)", "egs_fisher_host");
     return EGS_ERR_INVALID;
   }
-  // the augmented problem: 2 np rows, tile ts
-  egs_problem* probe = nullptr;
-  int rc = egs_problem_create(&probe, n, dts);
+  egs_problem* p = nullptr;
+  int rc = egs_problem_create(&p, n, dts);
   if (rc != EGS_OK) return rc;
-  int nn = 0, ts = 0, nt = 0;
-  long long bytes = 0;
-  egs_problem_info(probe, &nn, &ts, &nt, &bytes);
-  egs_problem_destroy(probe);
-  const long long np = (long long)nt * ts;
-  egs_problem* aug = nullptr;
-  if ((rc = egs_problem_create(&aug, (int)(2 * np), ts)) != EGS_OK) return rc;
-  std::unique_ptr<egs_problem, int (*)(egs_problem*)> guard(aug, egs_problem_destroy);
-  double* tiles = nullptr;
-  int ts2 = 0, nt2 = 0;
+  std::unique_ptr<egs_problem, int (*)(egs_problem*)> guard(p, egs_problem_destroy);
+  double *tiles = nullptr, *dx = nullptr, *dy = nullptr;
+  int ts = 0, nt = 0;
   cudaStream_t st = nullptr;
-  problem_tiles(aug, &tiles, &ts2, &nt2, &st);
-  if (ts2 != ts || nt2 != 2 * nt) {
-    set_last_error("unexpected augmented layout", "egs_fisher_host");
+  problem_tiles(p, &tiles, &dx, &dy, &ts, &nt, &st);
+  if (lower_tiles(2 * nt) > 65535) {
+    set_last_error("more than 180 tile rows; use a larger dts", "egs_fisher_host");
     return EGS_ERR_INVALID;
   }
-  const long long nn2 = np * np;
-  double *dx = nullptr, *dy = nullptr, *C = nullptr, *D = nullptr, *M = nullptr, *part = nullptr, *dots = nullptr;
-  const int nblk = 1184;
+  if ((rc = egs_problem_set_locations(p, x, y)) != EGS_OK || (rc = factor_resident(p, theta)) != EGS_OK) return rc;
+  const int np = nt * ts;
+  const size_t nn3 = 3 * (size_t)np * np;
+  double *Y = nullptr, *X = nullptr, *tabs = nullptr, *part = nullptr, *dots = nullptr;
+  MaternParams* orders = nullptr;
+  const int nblk = 296;
   auto cleanup = [&]() {
     cudaStreamSynchronize(st);
-    for (void* b : {(void*)dx, (void*)dy, (void*)C, (void*)D, (void*)M, (void*)part, (void*)dots}) cudaFreeAsync(b, st);
+    for (void* b : {(void*)Y, (void*)X, (void*)tabs, (void*)orders, (void*)part, (void*)dots}) cudaFreeAsync(b, st);
     cudaStreamSynchronize(st);
   };
-  if (cudaMallocAsync(&dx, np * sizeof(double), st) || cudaMallocAsync(&dy, np * sizeof(double), st) ||
-      cudaMallocAsync(&C, nn2 * sizeof(double), st) || cudaMallocAsync(&D, 3 * nn2 * sizeof(double), st) ||
-      cudaMallocAsync(&M, 3 * nn2 * sizeof(double), st) || cudaMallocAsync(&part, nblk * sizeof(double), st) ||
-      cudaMallocAsync(&dots, 9 * sizeof(double), st)) {
+  static std::once_flag tab_attr[64];
+  once_per_device(tab_attr, []() {
+    cudaFuncSetAttribute(matern_derivatives_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFisherTabBytes);
+  });
+  if (cudaMallocAsync(&Y, nn3 * sizeof(double), st) || cudaMallocAsync(&X, nn3 * sizeof(double), st) ||
+      cudaMallocAsync(&tabs, kFisherTabBytes, st) ||
+      cudaMallocAsync(&orders, kFisherOrders * sizeof(MaternParams), st) ||
+      cudaMallocAsync(&part, kPairs * nblk * sizeof(double), st) ||
+      cudaMallocAsync(&dots, kPairs * sizeof(double), st)) {
     cudaGetLastError();
     cleanup();
     set_last_error("device allocation failed", "egs_fisher_host");
     return EGS_ERR_OOM;
   }
-  cudaMemsetAsync(dx, 0, np * sizeof(double), st);
-  cudaMemsetAsync(dy, 0, np * sizeof(double), st);
-  cudaMemcpyAsync(dx, x, n * sizeof(double), cudaMemcpyHostToDevice, st);
-  cudaMemcpyAsync(dy, y, n * sizeof(double), cudaMemcpyHostToDevice, st);
-  // C with identity padding, dense
-  cudaMemsetAsync(C, 0, nn2 * sizeof(double), st);
-  if ((rc = launch_matern_block(C, (int)np, n, n, dx, dy, dx, dy, mp, st)) != EGS_OK) {
-    cleanup();
-    return rc;
-  }
-  {
-    std::vector<double> one(1, 1.0);
-    for (long long r = n; r < np; ++r)
-      cudaMemcpyAsync(C + r * np + r, one.data(), sizeof(double), cudaMemcpyHostToDevice, st);
-    cudaStreamSynchronize(st);
-  }
   FisherParams q;
   q.sigma2 = theta[0];
   q.beta = theta[1];
   q.nu = theta[2];
-  q.ginv = 1.0 / std::tgamma(q.nu);
   q.con = 1.0 / (std::pow(2.0, q.nu - 1.0) * std::tgamma(q.nu));
   q.psi = digamma(q.nu);
-  matern_derivatives_kernel<<<(unsigned)((nn2 + 255) / 256), 256, 0, st>>>(dx, dy, n, (int)np, q, D);
-  const long long ntiles2 = lower_tiles(2 * nt);
-  if (ntiles2 > 65535) {
+  // every order as a general one (half-integers included: mu = -1/2); orders
+  // below 0 (nu < 6e-3) mean K_{-nu} = K_nu
+  const double h = kFisherStep;
+  const double order[kFisherOrders] = {q.nu,           q.nu + 1.0,     q.nu + h,       q.nu - h,
+                                       q.nu + 2.0 * h, q.nu - 2.0 * h, q.nu + 3.0 * h, q.nu - 3.0 * h};
+  MaternParams hp[kFisherOrders];
+  for (int o = 0; o < kFisherOrders; ++o) {
+    hp[o] = mp;
+    hp[o].nu = order[o];
+    hp[o].n = (int)std::floor(order[o] + 0.5);
+    hp[o].mu = order[o] - hp[o].n;
+    hp[o].kind = 2;
+    hp[o].table = q.nu + 1.0 <= kKtabMaxNu ? 1 : 0;
+  }
+  cudaMemcpyAsync(orders, hp, sizeof(hp), cudaMemcpyHostToDevice, st);
+  launch_matern_ktab(orders, tabs, kFisherOrders, st);
+  matern_derivatives_kernel<<<3 * gemm_num_sms(), 256, kFisherTabBytes, st>>>(dx, dy, n, np, q, orders, tabs, Y);
+  // Y = C_j -> X = C_j L^-T; Y = X^T = L^-1 C_j -> X = L^-1 C_j L^-T = M_j
+  if ((rc = launch_rows_forward(tiles, ts, nt, Y, X, 3LL * np, 3 * np, st)) != EGS_OK) {
     cleanup();
-    set_last_error("the augmented matrix has more than 65535 tiles; use a larger dts", "egs_fisher_host");
-    return EGS_ERR_INVALID;
+    return rc;
   }
-  const unsigned gx = (unsigned)std::min<long long>(64, ((long long)ts * ts + 255) / 256);
-  for (int j = 0; j < 3; ++j) {
-    // pass 1: B = C_j -> Y = C_j L^-T;  pass 2: B = Y^T = L^-1 C_j -> L^-1 C_j L^-T = M_j
-    for (int pass = 0; pass < 2; ++pass) {
-      const double* B = pass == 0 ? D + j * nn2 : M + j * nn2;
-      augment_tiles_kernel<<<dim3(gx, (unsigned)ntiles2), 256, 0, st>>>(tiles, ts, nt, C, B, pass);
-      if ((rc = enqueue_potrf_steps(aug, nt)) != EGS_OK) {
-        cleanup();
-        return rc;
-      }
-      extract_block_kernel<<<(unsigned)((nn2 + 255) / 256), 256, 0, st>>>(tiles, ts, nt, M + j * nn2);
-    }
+  transpose_stacked_kernel<<<dim3(np / 64, np / 64, 3), 256, 0, st>>>(X, np, Y);
+  if ((rc = launch_rows_forward(tiles, ts, nt, Y, X, 3LL * np, 3 * np, st)) != EGS_OK) {
+    cleanup();
+    return rc;
   }
-  for (int j = 0; j < 3; ++j)
-    for (int k = j; k < 3; ++k) {
-      dot_partial_kernel<<<nblk, 256, 0, st>>>(M + j * nn2, M + k * nn2, nn2, part);
-      sum_partials_kernel<<<1, 32, 0, st>>>(part, nblk, dots + 3 * j + k);
-    }
-  double h[9] = {};
-  cudaMemcpyAsync(h, dots, sizeof(h), cudaMemcpyDeviceToHost, st);
+  pair_dots_kernel<<<nblk, 256, 0, st>>>(X, np, part);
+  pair_sums_kernel<<<1, 32 * kPairs, 0, st>>>(part, nblk, dots);
+  double h6[kPairs] = {};
+  cudaMemcpyAsync(h6, dots, sizeof(h6), cudaMemcpyDeviceToHost, st);
   if (cudaStreamSynchronize(st) != cudaSuccess || cudaGetLastError() != cudaSuccess) {
     set_last_error("a CUDA call failed", "egs_fisher_host");
     cleanup();
@@ -306,8 +264,8 @@ extern "C" int egs_fisher_host(int n, int dts, const double* x, const double* y,
   cleanup();
   // A (3 x 3, symmetric) and its inverse through a Cholesky factorisation
   double A[3][3];
-  for (int j = 0; j < 3; ++j)
-    for (int k = j; k < 3; ++k) A[j][k] = A[k][j] = 0.5 * h[3 * j + k];
+  for (int j = 0, i = 0; j < 3; ++j)
+    for (int k = j; k < 3; ++k) A[j][k] = A[k][j] = 0.5 * h6[i++];
   double L[3][3] = {};
   for (int j = 0; j < 3; ++j) {
     double s = A[j][j];

@@ -312,25 +312,28 @@ __device__ __forceinline__ void step_subst16(double (&v)[16], const double* blk,
   }
 }
 
-// One warp: rows row0 .. row0+31 of block X, sub-block q: substitution against
-// L_qq, then the update of the later sub-blocks.
+// One warp: rows row0 .. row0 + 16 MB - 1 of block X (MB = 1: the upper lanes
+// repeat the lower ones), sub-block q: substitution against L_qq, then the update
+// of the later sub-blocks.
+template <int MB>
 __device__ __forceinline__ void step_rows(double* X, const double* D, const double* pinv, int q, int row0, int lane) {
-  double* xr = X + row0 + lane;
+  double* xr = X + row0 + (MB == 2 ? lane : lane & 15);
   {
     double v[16];
 #pragma unroll
     for (int j = 0; j < 16; ++j) v[j] = xr[(16 * q + j) * kStepLd];
     step_subst16(v, D + (16 * q) * kStepLd + 16 * q, pinv + 16 * q);
+    __syncwarp();
 #pragma unroll
     for (int j = 0; j < 16; ++j) xr[(16 * q + j) * kStepLd] = v[j];
   }
   __syncwarp();
   if (q == 3) return;
-  double a[2][8];
-  frag_a_neg(X, row0, 16 * q, lane, a[0]);
-  frag_a_neg(X, row0 + 16, 16 * q, lane, a[1]);
+  double a[MB][8];
+#pragma unroll
+  for (int m = 0; m < MB; ++m) frag_a_neg(X, row0 + 16 * m, 16 * q, lane, a[m]);
 #pragma unroll 1
-  for (int n0 = 16 * (q + 1); n0 < kStep; n0 += 16) block_update_16<2>(X, row0, n0, D, 16 * q, lane, a);
+  for (int n0 = 16 * (q + 1); n0 < kStep; n0 += 16) block_update_16<MB>(X, row0, n0, D, 16 * q, lane, a);
   __syncwarp();
 }
 
@@ -443,7 +446,7 @@ __device__ __forceinline__ void panel_step_body(double* __restrict__ sm, double*
   } else {
 #pragma unroll 1
     for (int s = 0; s < 4; ++s) {
-      if (s > 0 && rows_warp) step_rows(A + rc * kStepBlock, D, pinv, s - 1, 32 * half, lane);
+      if (s > 0 && rows_warp) step_rows<2>(A + rc * kStepBlock, D, pinv, s - 1, 32 * half, lane);
       cp_async_wait<0>();
       bar_sync_all();
     }
@@ -458,7 +461,7 @@ __device__ __forceinline__ void panel_step_body(double* __restrict__ sm, double*
   const int ntiles = 8 * ncol;
   double cv[4][4];
   if (warp < ntiles) step_load_c(tile_ptr(warp), ts, cv);
-  if (rows_warp) step_rows(A + rc * kStepBlock, D, pinv, 3, 32 * half, lane);
+  if (rows_warp) step_rows<2>(A + rc * kStepBlock, D, pinv, 3, 32 * half, lane);
   if (diag_warp == 1) z_substep(3);
   __syncthreads();
 

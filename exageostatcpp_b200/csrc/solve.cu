@@ -17,6 +17,7 @@
 // Reference counterparts: CHAMELEON_dtrsm_Tile / dposv on one vector
 // (ChameleonImplementation.cpp:337-347, LinearAlgebraMethods.cpp:544) and the
 // per-target solves of the MLOE / MMOM loop (LinearAlgebraMethods.cpp:802-1131).
+#include <algorithm>
 #include "common.cuh"
 #include "kernels.cuh"
 #include "panel_step.cuh"
@@ -204,11 +205,11 @@ __device__ __forceinline__ void frag_bt(const double* x, int n0, int k0, int lan
   for (int i = 0; i < 4; ++i) b[i] = x[(n0 + g) * kStepLd + k0 + t + 4 * i];
 }
 
-// One warp: rows row0 .. row0+31 of X, sub-block q (16 columns) of X := X L^-1:
-// substitution against L_qq from the last column down, then the update of the
-// earlier sub-blocks.
+// One warp: rows row0 .. row0+15 of X (the upper lanes repeat the lower ones),
+// sub-block q (16 columns) of X := X L^-1: substitution against L_qq from the
+// last column down, then the update of the earlier sub-blocks.
 __device__ __forceinline__ void rows_back16(double* X, const double* D, const double* pinv, int q, int row0, int lane) {
-  double* xr = X + row0 + lane;
+  double* xr = X + row0 + (lane & 15);
   const double* blk = D + (16 * q) * kStepLd + 16 * q;
   {
     double v[16];
@@ -222,31 +223,29 @@ __device__ __forceinline__ void rows_back16(double* X, const double* D, const do
       for (int c = 0; c < 16; ++c)
         if (c < j) v[c] = fma(-v[j], blk[c * kStepLd + j], v[c]);
     }
+    __syncwarp();
 #pragma unroll
     for (int j = 0; j < 16; ++j) xr[(16 * q + j) * kStepLd] = v[j];
   }
   __syncwarp();
   if (q == 0) return;
-  double a[2][8];
-  frag_a_neg(X, row0, 16 * q, lane, a[0]);
-  frag_a_neg(X, row0 + 16, 16 * q, lane, a[1]);
-#pragma unroll 1
+  double a[8];
+  frag_a_neg(X, row0, 16 * q, lane, a);
+#pragma unroll 2
   for (int n0 = 0; n0 < 16 * q; n0 += 8) {
-    double b[4], c[2][4];
+    double b[4], c[4];
     frag_bt(D, n0, 16 * q, lane, b);  // rows 16 q .. of columns n0 ..
-#pragma unroll
-    for (int m = 0; m < 2; ++m) {
-      frag_c_load(X, row0 + 16 * m, n0, lane, c[m]);
-      dmma_16816(c[m], a[m], b);
-      frag_c_store(X, row0 + 16 * m, n0, lane, c[m]);
-    }
+    frag_c_load(X, row0, n0, lane, c);
+    dmma_16816(c, a, b);
+    frag_c_store(X, row0, n0, lane, c);
   }
   __syncwarp();
 }
 
 // Step of the 64 columns at global column r0 = k ts + kb: X_b := Y_b L_bb^-T (kBack:
 // L_bb^-1) for the 64 rows 64 blockIdx.y .., and Y_j -= X_b L_jb^T (kBack: X_b L_bj) for
-// the column block j of blockIdx.x.  Y and X are column-major with column stride ldy.
+// the column blocks j = blockIdx.x, blockIdx.x + gridDim.x, .. of the nblk remaining
+// ones.  Y and X are column-major with column stride ldy.
 template <bool kBack>
 __global__ void __launch_bounds__(kRowsThreads)
 rows_step_kernel(const double* __restrict__ tiles, int ts, int nt, int k, int kb, int nblk, double* Y,
@@ -256,31 +255,29 @@ rows_step_kernel(const double* __restrict__ tiles, int ts, int nt, int k, int kb
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const long long ts2 = (long long)ts * ts;
   const int r0 = k * ts + kb;
-  const bool have = (int)blockIdx.x < nblk;
-  const int at = kBack ? kStep * blockIdx.x : r0 + kStep * (blockIdx.x + 1);  // column block j
   double* Yc = Y + kStep * blockIdx.y;
-  load_block(D, tiles + tile_slot(k, k, nt) * ts2 + (long long)kb * ts + kb, ts, kRowsThreads);
-  load_block(A, Yc + r0 * ldy, ldy, kRowsThreads);
-  cp_async_commit();
-  if (have) {
-    const int t = at / ts, lo = at - t * ts;
+  auto first_col = [&](int j) { return kBack ? kStep * j : r0 + kStep * (j + 1); };
+  auto fetch_b = [&](int j) {
+    const int at = first_col(j), t = at / ts, lo = at - t * ts;
     load_block(B, tiles + (kBack ? tile_slot(k, t, nt) * ts2 + (long long)lo * ts + kb
                                  : tile_slot(t, k, nt) * ts2 + (long long)kb * ts + lo),
                ts, kRowsThreads);
-  }
+  };
+  load_block(D, tiles + tile_slot(k, k, nt) * ts2 + (long long)kb * ts + kb, ts, kRowsThreads);
+  load_block(A, Yc + r0 * ldy, ldy, kRowsThreads);
+  cp_async_commit();
+  if ((int)blockIdx.x < nblk) fetch_b(blockIdx.x);
   cp_async_commit();
   cp_async_wait<1>();
   __syncthreads();
   if (tid < kStep) pinv[tid] = 1.0 / D[tid * kStepLd + tid];
   __syncthreads();
-  if (warp < 2) {
 #pragma unroll 1
-    for (int u = 0; u < 4; ++u) {
-      if constexpr (kBack) {
-        rows_back16(A, D, pinv, 3 - u, 32 * warp, lane);
-      } else {
-        step_rows(A, D, pinv, u, 32 * warp, lane);
-      }
+  for (int u = 0; u < 4; ++u) {
+    if constexpr (kBack) {
+      rows_back16(A, D, pinv, 3 - u, 16 * warp, lane);
+    } else {
+      step_rows<1>(A, D, pinv, u, 16 * warp, lane);
     }
   }
   cp_async_wait<0>();
@@ -292,33 +289,42 @@ rows_step_kernel(const double* __restrict__ tiles, int ts, int nt, int k, int kb
       *reinterpret_cast<double2*>(Xc + (r0 + c) * ldy + r) = *reinterpret_cast<const double2*>(A + c * kStepLd + r);
     }
   }
-  if (!have) return;
   const int g = lane >> 2, t = lane & 3;
 #pragma unroll 1
-  for (int n2 = 0; n2 < 2; ++n2) {
-    double* p = Yc + (long long)(at + 32 * n2 + 2 * t) * ldy + 16 * warp + 2 * g;
-    double c[4][4];
+  for (int j = blockIdx.x; j < nblk; j += gridDim.x) {
+    if (j != (int)blockIdx.x) {
+      __syncthreads();  // every warp is done with the previous block of L
+      fetch_b(j);
+      cp_async_commit();
+    }
+    // this warp's 16 rows of Y_j, under way together with the block of L
+    double* p = Yc + (long long)(first_col(j) + 2 * t) * ldy + 16 * warp + 2 * g;
+    double c[8][4];
 #pragma unroll
-    for (int ni = 0; ni < 4; ++ni)
+    for (int ni = 0; ni < 8; ++ni)
 #pragma unroll
       for (int h = 0; h < 2; ++h) ldg_v2f64(p + (8 * ni + h) * ldy, c[ni][h], c[ni][2 + h]);
+    if (j != (int)blockIdx.x) {
+      cp_async_wait<0>();
+      __syncthreads();
+    }
 #pragma unroll
     for (int kk = 0; kk < 4; ++kk) {
       double a[8];
       frag_a_neg(A, 16 * warp, 16 * kk, lane, a);
 #pragma unroll
-      for (int ni = 0; ni < 4; ++ni) {
+      for (int ni = 0; ni < 8; ++ni) {
         double b[4];
         if constexpr (kBack) {
-          frag_bt(B, 32 * n2 + 8 * ni, 16 * kk, lane, b);
+          frag_bt(B, 8 * ni, 16 * kk, lane, b);
         } else {
-          frag_b(B, 32 * n2 + 8 * ni, 16 * kk, lane, b);
+          frag_b(B, 8 * ni, 16 * kk, lane, b);
         }
         dmma_16816(c[ni], a, b);
       }
     }
 #pragma unroll
-    for (int ni = 0; ni < 4; ++ni)
+    for (int ni = 0; ni < 8; ++ni)
 #pragma unroll
       for (int h = 0; h < 2; ++h) stg_v2f64(p + (8 * ni + h) * ldy, c[ni][h], c[ni][2 + h]);
   }
@@ -404,6 +410,25 @@ rows_dot_kernel(const double* __restrict__ A, const double* __restrict__ B, long
 constexpr int rows_step_smem() { return (3 * kStepBlock + kStep) * (int)sizeof(double); }
 constexpr int rows_times_smem() { return 4 * kStepBlock * (int)sizeof(double); }
 
+// Column blocks per CTA of a step with nblk of them and `chunks` row chunks: a
+// CTA's own solve costs about 1.25 block updates and two CTAs fit an SM, so the
+// cheapest split has few partial waves (Fisher information N = 1,600, 75 chunks:
+// 40.6 us a step on average, 47 with at most four blocks per CTA).
+int rows_share(int nblk, int chunks) {
+  const long long slots = 2LL * gemm_num_sms();
+  int best = 1;
+  double cost = 1e300;
+  for (int share = 1; share <= 16 && share <= nblk; ++share) {
+    const long long ctas = (long long)((nblk + share - 1) / share) * chunks;
+    const double c = (double)((ctas + slots - 1) / slots) * (1.25 + share);
+    if (c < cost) {
+      cost = c;
+      best = share;
+    }
+  }
+  return best;
+}
+
 template <bool kBack>
 int rows_solve(const double* tiles, int ts, int nt, double* Y, double* X, long long ldy, int rows, cudaStream_t st) {
   static std::once_flag done[64];
@@ -417,8 +442,9 @@ int rows_solve(const double* tiles, int ts, int nt, double* Y, double* X, long l
   for (int i = 0; i < steps; ++i) {
     const int b = kBack ? steps - 1 - i : i;
     const int nblk = kBack ? b : steps - 1 - b;
-    rows_step_kernel<kBack><<<dim3(nblk > 0 ? nblk : 1, rows / kStep), kRowsThreads, rows_step_smem(), st>>>(
-        tiles, ts, nt, b / per, (b % per) * kStep, nblk, Y, X, ldy);
+    const int share = rows_share(nblk, rows / kStep);
+    rows_step_kernel<kBack><<<dim3(nblk > 0 ? (nblk + share - 1) / share : 1, rows / kStep), kRowsThreads,
+                              rows_step_smem(), st>>>(tiles, ts, nt, b / per, (b % per) * kStep, nblk, Y, X, ldy);
   }
   return launch_status("rows_step_kernel");
 }

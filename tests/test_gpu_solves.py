@@ -53,3 +53,19 @@ def test_mloe_mmom_reports_a_failing_covariance():
     x[17], y[17] = x[16], y[16]
     with pytest.raises(egs.NotPositiveDefinite):
         egs.mloe_mmom_host(x[:90], y[:90], x[90:], y[90:], (1.0, 0.05, 1.5), (0.8, 0.06, 1.5), 64)
+
+
+@pytest.mark.parametrize("n,dts,theta", [(1, 64, (1.0, 0.1, 0.5)), (64, 64, (1.0, 0.05, 1.5)), (65, 64, (0.7, 0.05, 0.3)),
+                                         (500, 192, (1.2, 0.03, 1.0)), (700, 320, (1.0, 0.002, 0.8)),
+                                         (300, 128, (1.0, 0.02, 6.9)), (300, 128, (1.0, 0.015, 7.5))])
+def test_fisher_orders_and_sizes(n, dts, theta):
+    # beta = 0.002 puts distances beyond the tables, nu + 1 > 8 turns them off;
+    # 1e-7 is the bound of the Richardson derivative in the other Fisher tests
+    x, y = egs.generate_locations(n, 9)
+    if n == 1:  # one point: no information on beta and nu
+        with pytest.raises(egs.EgsError):
+            egs.fisher_host(x, y, theta, dts)
+        return
+    inv = egs.fisher_host(x, y, theta, dts)
+    ref = O.fisher_inverse(x, y, theta)
+    assert np.abs(inv - ref).max() <= 1e-7 * np.abs(ref).max(), (inv, ref)
