@@ -70,3 +70,43 @@ inline int launch_status(const char* where) {
   return EGS_ERR_CUDA;
 }
 }
+
+namespace egs {
+
+// Programmatic dependent launch.  A kernel launched with launch_overlapped may
+// start before the previous kernel of its stream has ended; every one of its
+// blocks calls grid_dependency_wait() before it touches memory (and before it
+// returns), which waits for the end of all earlier work.  A kernel calls
+// grid_dependents_launch() towards its end to let the next such kernel's launch
+// and set-up overlap with its tail.  Both are no-ops for ordinary launches.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependents_launch() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <typename T>
+struct same_type {
+  using type = T;
+};
+
+template <typename... P>
+inline int launch_overlapped(const char* where, void (*kern)(P...), dim3 grid, dim3 block, size_t smem,
+                             cudaStream_t st, typename same_type<P>::type... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, args...);
+  if (e == cudaSuccess) return EGS_OK;
+  cudaGetLastError();
+  set_last_error(cudaGetErrorString(e), where);
+  return EGS_ERR_CUDA;
+}
+
+}  // namespace egs

@@ -133,7 +133,7 @@ dgemm_update_kernel(const __grid_constant__ CUtensorMap tmap, double* __restrict
   using S = Shape<CFG>;
   constexpr int BM = S::BM, BN = S::BN, STAGES = S::STAGES;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  // the job of this block, and its tile
+  // the job of this block, and its tile (job tables are constant)
   const GemmDesc* dp = &single;
   long long L = blockIdx.x;
   if constexpr (kBatched) {
@@ -148,7 +148,10 @@ dgemm_update_kernel(const __grid_constant__ CUtensorMap tmap, double* __restrict
   const GemmDesc& d = *dp;
   int mb, nb;
   decode_block(L, d, mb, nb);
-  if (block_skipped(d, mb, nb)) return;
+  if (block_skipped(d, mb, nb)) {
+    grid_dependency_wait();
+    return;
+  }
   // 1024-byte aligned stage base (128B-swizzle atoms), kept as an offset into the
   // shared array so every access stays a shared-memory access.
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -164,6 +167,7 @@ dgemm_update_kernel(const __grid_constant__ CUtensorMap tmap, double* __restrict
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   __syncthreads();
+  grid_dependency_wait();
   const int ksteps = d.K / BK;
 
   // Producer state: lane b of warp 0 loads box b of every stage (A boxes first).
@@ -279,6 +283,7 @@ dgemm_update_kernel(const __grid_constant__ CUtensorMap tmap, double* __restrict
     return;
   }
 
+  grid_dependents_launch();
   // Epilogue: C -= acc; element pairs (row, row+1) are contiguous in a column.
   // Per n8 block all loads are issued before any store.
   long long rp[S::MI];
@@ -407,13 +412,20 @@ static int launch_cfg(int cfg, const void* tmap, double* tiles, const GemmDesc& 
   using namespace gemm;
   set_gemm_smem_attributes();
   const CUtensorMap& tm = *reinterpret_cast<const CUtensorMap*>(tmap);
-  if (cfg == 0)
-    dgemm_update_kernel<0, kBatched><<<(unsigned)total, THREADS, Shape<0>::SMEM_BYTES, st>>>(tm, tiles, d, J, err);
-  else if (cfg == 2)
-    dgemm_update_kernel<2, kBatched><<<(unsigned)total, THREADS, Shape<2>::SMEM_BYTES, st>>>(tm, tiles, d, J, err);
-  else
-    dgemm_update_kernel<1, kBatched><<<(unsigned)total, THREADS, Shape<1>::SMEM_BYTES, st>>>(tm, tiles, d, J, err);
-  return launch_status("dgemm_update_kernel");
+  const char* where = "dgemm_update_kernel";
+  const dim3 grid((unsigned)total), block(THREADS);
+  if (cfg == 0) {
+    dgemm_update_kernel<0, kBatched><<<grid, block, Shape<0>::SMEM_BYTES, st>>>(tm, tiles, d, J, err);
+    return launch_status(where);
+  }
+  // Small launches overlap their set-up with the tail of the panel step before
+  // them (N = 1,600: 605 -> 582 us per evaluation); large ones, and the panel steps
+  // themselves, only take room from the tail they wait for (N = 10,000: 15.9 -> 16.1 ms).
+  if (cfg == 1)
+    return launch_overlapped(where, dgemm_update_kernel<1, kBatched>, grid, block, Shape<1>::SMEM_BYTES, st, tm, tiles,
+                             d, J, err);
+  return launch_overlapped(where, dgemm_update_kernel<2, kBatched>, grid, block, Shape<2>::SMEM_BYTES, st, tm, tiles, d,
+                           J, err);
 }
 
 static int launch_desc(const void* tmap, double* tiles, GemmDesc& d, int* err, cudaStream_t st) {

@@ -465,6 +465,7 @@ __device__ __forceinline__ void panel_step_body(double* __restrict__ sm, double*
   if (diag_warp == 1) z_substep(3);
   __syncthreads();
 
+  grid_dependents_launch();
   // solved rows out
   if (chunk >= 0) {
     double* dst = inner ? out + kStep * (chunk + 1) : own + (long long)kb * ts;

@@ -38,6 +38,8 @@ panel_step_kernel(double* col, int ts, int nchunk, int kb, int nb, int gcol, int
 
 __global__ void __launch_bounds__(kStepThreads)
 panel_flush_kernel(const double* __restrict__ slot, double* __restrict__ col, int ts, int kb, double* __restrict__ z) {
+  grid_dependents_launch();
+  grid_dependency_wait();
   panel_flush_body(slot, col, ts, kb, blockIdx.x, z);
 }
 
@@ -82,9 +84,10 @@ int launch_panel_step(double* col, int ts, int rows_below, int kb, int nb, int g
 int launch_panel_flush(PanelChain& ch, cudaStream_t st) {
   if (ch.chunks == 0) return EGS_OK;
   const double* slot = ch.scratch + (long long)(ch.parity ^ 1) * kScratchSlot;
-  panel_flush_kernel<<<ch.chunks, kStepThreads, 0, st>>>(slot, ch.col, ch.ts, ch.kb, ch.z);
+  const int chunks = ch.chunks;
   ch.chunks = 0;
-  return launch_status("panel_flush_kernel");
+  return launch_overlapped("panel_flush_kernel", panel_flush_kernel, dim3(chunks), dim3(kStepThreads), 0, st, slot,
+                           ch.col, ch.ts, ch.kb, ch.z);
 }
 
 // ---------------------------------------------------------------------------
@@ -95,24 +98,28 @@ __global__ void __launch_bounds__(256)
 logdet_partials_kernel(const double* __restrict__ tiles, int ts, int nt, int n, double* __restrict__ partial) {
   const int k = blockIdx.x;
   const int rows = min(ts, n - k * ts);
+  grid_dependents_launch();
+  grid_dependency_wait();
   const double s = logdet_tile_body(tiles + tile_slot(k, k, nt) * (long long)ts * ts, ts, rows);
   if (threadIdx.x == 0) partial[k] = s;
 }
 
 void launch_logdet_partials(const double* tiles, int ts, int nt, int n, double* partial, cudaStream_t st) {
-  logdet_partials_kernel<<<nt, 256, 0, st>>>(tiles, ts, nt, n, partial);
+  launch_overlapped("logdet_partials_kernel", logdet_partials_kernel, dim3(nt), dim3(256), 0, st, tiles, ts, nt, n,
+                    partial);
 }
 
 // result = (log-likelihood, log|C|, Z^T C^-1 Z after the solve, info) (finalize_body).
 __global__ void __launch_bounds__(256)
 finalize_kernel(const double* __restrict__ partial, int nt, const double* __restrict__ z, int n,
                 double* __restrict__ result, const int* __restrict__ info) {
+  grid_dependency_wait();
   finalize_body(partial, nt, z, n, result, info);
 }
 
 void launch_finalize(const double* partial, int nt, const double* z, int n, double* result, const int* info,
                      cudaStream_t st) {
-  finalize_kernel<<<1, 256, 0, st>>>(partial, nt, z, n, result, info);
+  launch_overlapped("finalize_kernel", finalize_kernel, dim3(1), dim3(256), 0, st, partial, nt, z, n, result, info);
 }
 
 // out[0] = sum (a - b)^2 (DMSECodelet, dmse-codelet.cpp:60-73), fixed order.

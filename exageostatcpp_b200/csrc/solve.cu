@@ -28,13 +28,6 @@ namespace {
 
 constexpr int kVecThreads = 256;
 
-// Waits for the previous launch of the stream when this one was allowed to
-// start before its end (a no-op otherwise), and lets the next one start.
-__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_dependents_launch() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-
 // The 64 x 64 block at `src` (column stride ts) into shared memory.
 __device__ __forceinline__ void load_block(double* dst, const double* src, long long ld, int threads) {
   for (int e = threadIdx.x; e < kStep * kStep / 2; e += threads) {
@@ -155,24 +148,6 @@ __global__ void vec_last_kernel(const double* __restrict__ prev, double* __restr
   pz[threadIdx.x] = prev[threadIdx.x];
 }
 
-// Launches `kern` so that it may start before the previous launch of the stream
-// has ended (overlap: it waits by itself) or after it.
-template <typename... P, typename... Q>
-int launch_dependent(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool overlap, Q... args) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = overlap ? 1 : 0;
-  if (cudaLaunchKernelEx(&cfg, kern, P(args)...) != cudaSuccess) return launch_status("launch_dependent");
-  return EGS_OK;
-}
-
 template <bool kBack>
 int vec_solve(const double* tiles, int ts, int nt, double* z, double* scratch, cudaStream_t st, long long* launches) {
   const int per = ts / kStep, steps = nt * per;
@@ -183,14 +158,21 @@ int vec_solve(const double* tiles, int ts, int nt, double* z, double* scratch, c
     const int nblk = kBack ? b : steps - 1 - b;
     double* out = scratch + (i & 1) * kStep;
     // the first step starts after whatever wrote the factor
-    const int rc = launch_dependent(vec_step_kernel<kBack>, dim3(nblk > 0 ? nblk : 1), dim3(kVecThreads), 0, st, i > 0,
-                                    tiles, ts, nt, b / per, (b % per) * kStep, nblk, z, out, prev, pz);
+    int rc = EGS_OK;
+    if (i == 0) {
+      vec_step_kernel<kBack><<<nblk > 0 ? nblk : 1, kVecThreads, 0, st>>>(tiles, ts, nt, b / per, (b % per) * kStep,
+                                                                          nblk, z, out, prev, pz);
+      rc = launch_status("vec_step_kernel");
+    } else {
+      rc = launch_overlapped("vec_step_kernel", vec_step_kernel<kBack>, dim3(nblk > 0 ? nblk : 1), dim3(kVecThreads),
+                             0, st, tiles, ts, nt, b / per, (b % per) * kStep, nblk, z, out, prev, pz);
+    }
     if (rc != EGS_OK) return rc;
     prev = out;
     pz = z + (long long)b * kStep;
   }
   *launches += steps + 1;
-  return launch_dependent(vec_last_kernel, dim3(1), dim3(kStep), 0, st, true, prev, pz);
+  return launch_overlapped("vec_last_kernel", vec_last_kernel, dim3(1), dim3(kStep), 0, st, prev, pz);
 }
 
 // ---------------------------------------------------------------------------
