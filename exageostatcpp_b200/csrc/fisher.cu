@@ -202,23 +202,26 @@ extern "C" int egs_fisher_host(int n, int dts, const double* x, const double* y,
   const int nblk = 296;
   auto cleanup = [&]() {
     cudaStreamSynchronize(st);
-    for (void* b : {(void*)Y, (void*)X, (void*)tabs, (void*)orders, (void*)part, (void*)dots}) cudaFreeAsync(b, st);
+    for (void* b : {(void*)Y, (void*)X, (void*)tabs, (void*)orders, (void*)part, (void*)dots})
+      if (b) cudaFreeAsync(b, st);
     cudaStreamSynchronize(st);
   };
   static std::once_flag tab_attr[64];
   once_per_device(tab_attr, []() {
     cudaFuncSetAttribute(matern_derivatives_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFisherTabBytes);
   });
-  if (cudaMallocAsync(&Y, nn3 * sizeof(double), st) || cudaMallocAsync(&X, nn3 * sizeof(double), st) ||
-      cudaMallocAsync(&tabs, kFisherTabBytes, st) ||
-      cudaMallocAsync(&orders, kFisherOrders * sizeof(MaternParams), st) ||
-      cudaMallocAsync(&part, kPairs * nblk * sizeof(double), st) ||
-      cudaMallocAsync(&dots, kPairs * sizeof(double), st)) {
-    cudaGetLastError();
-    cleanup();
-    set_last_error("device allocation failed", "egs_fisher_host");
-    return EGS_ERR_OOM;
-  }
+  const struct {
+    void** p;
+    size_t bytes;
+  } bufs[] = {{(void**)&Y, nn3 * sizeof(double)},      {(void**)&X, nn3 * sizeof(double)},
+              {(void**)&tabs, (size_t)kFisherTabBytes}, {(void**)&orders, kFisherOrders * sizeof(MaternParams)},
+              {(void**)&part, kPairs * nblk * sizeof(double)}, {(void**)&dots, kPairs * sizeof(double)}};
+  for (const auto& b : bufs)
+    if (alloc_from_pool(b.p, b.bytes, st) != EGS_OK) {
+      cleanup();
+      set_last_error("device allocation failed", "egs_fisher_host");
+      return EGS_ERR_OOM;
+    }
   FisherParams q;
   q.sigma2 = theta[0];
   q.beta = theta[1];

@@ -7,6 +7,9 @@
 
 namespace egs {
 
+// Stream-ordered device memory from the library's pool (capi.cu); released with cudaFreeAsync.
+int alloc_from_pool(void** p, size_t bytes, cudaStream_t st);
+
 int make_matern_params(const double* theta, MaternParams* out);
 // Builds the Chebyshev table of K_nu for theta (ktab: kKtabDoubles device
 // doubles), then generates every lower tile.
