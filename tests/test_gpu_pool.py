@@ -1,5 +1,6 @@
 """The library's memory pool: what it keeps is bounded, reused memory changes no
 result (bit for bit), and several threads can create and destroy problems."""
+import functools
 import threading
 
 import numpy as np
@@ -13,8 +14,13 @@ pytestmark = pytest.mark.gpu
 KEEP = 1 << 30
 
 
+@functools.lru_cache(None)
+def _points(n):  # the generator draws from the process-wide rand(): main thread only
+    return egs.generate_locations(n, 3)
+
+
 def _eval(n, dts, mixed=False):
-    x, y = egs.generate_locations(n, 3)
+    x, y = _points(n)
     p = egs.Problem(n, dts)
     if mixed:
         p.set_precision(egs.EGS_PRECISION_MIXED, 1)
