@@ -43,7 +43,7 @@ matern_batch_kernel(double* __restrict__ tiles, const double* __restrict__ x, co
                     const int4* __restrict__ tinfo, long long t0, int ts, const MaternParams* __restrict__ params,
                     const double* __restrict__ ktab, const long long* __restrict__ loc_base,
                     const int* __restrict__ nvec) {
-  __shared__ double stab[kKtabDoubles];
+  __shared__ __align__(16) double stab[kKtabShared];
   const long long t = t0 + blockIdx.y;
   const int4 ti = tinfo[t];
   const int p = ti.x;

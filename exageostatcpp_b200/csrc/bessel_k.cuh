@@ -187,7 +187,7 @@ __device__ __forceinline__ double matern_positive(double x, const MaternParams& 
 }
 
 // ---------------------------------------------------------------------------
-// Piecewise Chebyshev table of g(x) = e^x x^nu K_nu(x) for general nu.
+// Piecewise polynomial table of g(x) = e^x x^nu K_nu(x) for general nu.
 //
 // For one theta the generator evaluates the same K_nu at millions of distances;
 // the series/continued-fraction evaluation above costs thousands of FP64
@@ -200,14 +200,22 @@ __device__ __forceinline__ double matern_positive(double x, const MaternParams& 
 // (3 + 2 sqrt2) half-widths from each interval's centre, so the series
 // converge like (5.83 + sqrt(5.83^2 - 1))^-k ~ 11.6^-k: the interpolant is
 // within a few 1e-15 (relative) of g for nu <= 8 (checked against 30-digit
-// values).  An element then costs one table lookup, a 16-term Clenshaw sum and
-// one exp.  Distances outside [2^-20, 2^9) and nu > 8 use the direct
-// evaluation.
+// values).  The series are stored as powers of the local coordinate t (the
+// powers' coefficients of T_k grow like (1 + sqrt2)^k, far slower than the
+// series falls, so nothing cancels): an element then costs one table lookup, 15
+// fused multiply-adds and one exp.  Its row loads, which differ between the
+// lanes, and the root, quotient and exp bound it about equally: N = 40,000, nu =
+// 0.8, 5.5 ms (145e9 elements/s), 6.9 with a Clenshaw sum, the division and a 64-bit
+// index division per pair.  A table of x^nu K_nu(x) in x^2, which needs none of
+// the three, reached 4.8 ms but lost one to two digits where K falls steeply.
+// Distances outside [2^-20, 2^9) and nu > 8 use the direct evaluation.
 constexpr int kKtabDeg = 16;     // coefficients per interval
-constexpr int kKtabStride = 17;  // padded row: lanes reading different intervals hit different banks
+constexpr int kKtabStride = 17;  // doubles per interval in device memory
+constexpr int kKtabRow = 18;     // doubles per interval in shared memory (16-byte rows)
 constexpr int kKtabELo = -20, kKtabEHi = 9;
 constexpr int kKtabIntervals = 2 * (kKtabEHi - kKtabELo);
 constexpr int kKtabDoubles = kKtabIntervals * kKtabStride;
+constexpr int kKtabShared = kKtabIntervals * kKtabRow;
 constexpr double kKtabMaxNu = 8.0;
 // t = x * 2^-e * S_h + C maps interval (e, h) onto [-1, 1]:
 // h = 0: S = 2 / (sqrt2 - 1) = 2 + 2 sqrt2; h = 1: S = 2 + sqrt2; C = -(3 + 2 sqrt2) for both.
@@ -243,17 +251,18 @@ __device__ __forceinline__ double ktab_node(int idx, int j) {
   return (t - kKtabC) / (h ? kKtabS1 : kKtabS0) * scale;
 }
 
-// Clenshaw sum of one interval's Chebyshev series at t.
+// One interval's polynomial at t (Horner); c is a 16-byte aligned row in shared memory.
 __device__ __forceinline__ double ktab_sum(const double* __restrict__ c, double t) {
-  const double t2 = 2.0 * t;
-  double b1 = 0.0, b2 = 0.0;
+  const double2* c2 = reinterpret_cast<const double2*>(c);
+  double2 v = c2[kKtabDeg / 2 - 1];
+  double s = fma(v.y, t, v.x);
 #pragma unroll
-  for (int k = kKtabDeg - 1; k >= 1; --k) {
-    const double b0 = fma(t2, b1, c[k] - b2);
-    b2 = b1;
-    b1 = b0;
+  for (int k = kKtabDeg / 2 - 2; k >= 0; --k) {
+    v = c2[k];
+    s = fma(s, t, v.y);
+    s = fma(s, t, v.x);
   }
-  return fma(t, b1, c[0] - b2);
+  return s;
 }
 
 // Euclidean distance sqrt(dx^2 + dy^2) with dx = x2 - x1, dy = y2 - y1, rounded
@@ -272,16 +281,22 @@ __device__ __forceinline__ double matern_from_dist(double dist, const MaternPara
   return (x == 0.0) ? p.sigma2 : matern_positive(x, p);
 }
 
-// The same entry through the Chebyshev table tab (kKtabDoubles, any address
-// space) when p.table is set.
-__device__ __forceinline__ double matern_from_dist_tab(double dist, const MaternParams& p,
+// The same entry through the polynomial table tab (kKtabShared doubles of shared
+// memory) when p.table is set.  rbeta is 1 / beta, correctly rounded: the quotient
+// dist / beta is then one product and one correction by its exact residual
+// (Markstein: the result is the correctly rounded quotient).  Products that
+// over- or underflow give an x outside the table and take the division.
+__device__ __forceinline__ double matern_from_dist_tab(double dist, const MaternParams& p, double rbeta,
                                                        const double* __restrict__ tab) {
-  const double x = __ddiv_rn(dist, p.beta);
-  if (x == 0.0) return p.sigma2;
+  double x = dist * rbeta;
+  x = fma(fma(-x, p.beta, dist), rbeta, x);
   int idx;
   double t;
-  if (p.table && ktab_locate(x, idx, t)) return p.con * (ktab_sum(tab + idx * kKtabStride, t) * exp(-x));
-  return matern_positive(x, p);
+  if (ktab_locate(x, idx, t)) {
+    if (p.table) return p.con * (ktab_sum(tab + idx * kKtabRow, t) * exp(-x));
+    return matern_positive(x, p);
+  }
+  return matern_from_dist(dist, p);
 }
 
 }  // namespace egs

@@ -1820,9 +1820,8 @@ int egs_predict_host(int n_obs, int n_miss, int dts, const double* x_obs, const 
     cleanup();
     return EGS_ERR_CUDA;
   }
-  MaternParams mp;
-  make_matern_params(theta, &mp);
-  if ((rc = launch_matern_block(c12t, n_obs, n_obs, n_miss, p->x, p->y, dxm, dym, mp, st)) != EGS_OK) {
+  if ((rc = launch_matern_block_tab(c12t, n_obs, n_obs, n_miss, p->x, p->y, dxm, dym, p->dparams, p->ktab, st)) !=
+      EGS_OK) {
     cleanup();
     return rc;
   }
@@ -1907,9 +1906,8 @@ int egs_problem_predict(egs_problem* p, const double* theta, int n_miss, const d
   }
   cudaMemcpyAsync(dxm, x_miss, n_miss * sizeof(double), cudaMemcpyHostToDevice, st);
   cudaMemcpyAsync(dym, y_miss, n_miss * sizeof(double), cudaMemcpyHostToDevice, st);
-  MaternParams mp;
-  make_matern_params(theta, &mp);
-  rc = launch_matern_block(c12t, p->n, p->n, n_miss, p->x, p->y, dxm, dym, mp, st);
+  // parameters and table of theta are those of the factorisation above
+  rc = launch_matern_block_tab(c12t, p->n, p->n, n_miss, p->x, p->y, dxm, dym, p->dparams, p->ktab, st);
   launch_gemv_t_block(c12t, p->n, p->n, n_miss, p->z, dzm, st);
   cudaMemcpyAsync(z_miss, dzm, n_miss * sizeof(double), cudaMemcpyDeviceToHost, st);
   if (rc == EGS_OK) rc = check_cuda("egs_problem_predict");
@@ -1990,8 +1988,10 @@ int egs_mloe_mmom_host(int n_obs, int n_miss, int dts, const double* x_obs, cons
     cudaMemsetAsync(ya, 0, 2 * block * sizeof(double), st);
     cudaMemsetAsync(yt, 0, block * sizeof(double), st);
     // k_a and k_t of every target (padding rows and columns stay 0)
-    if ((rc = launch_matern_block(ya, (int)lda, m, n_obs, xm, ym, pa->x, pa->y, ma, st)) != EGS_OK ||
-        (rc = launch_matern_block(ya + group, (int)lda, m, n_obs, xm, ym, pa->x, pa->y, mt, st)) != EGS_OK)
+    if ((rc = launch_matern_block_tab(ya, (int)lda, m, n_obs, xm, ym, pa->x, pa->y, pa->dparams, pa->ktab, st)) !=
+            EGS_OK ||
+        (rc = launch_matern_block_tab(ya + group, (int)lda, m, n_obs, xm, ym, pa->x, pa->y, pt->dparams, pt->ktab,
+                                      st)) != EGS_OK)
       break;
     cudaMemcpy2DAsync(yt, ldt * sizeof(double), ya + group, lda * sizeof(double), ldt * sizeof(double), np,
                       cudaMemcpyDeviceToDevice, st);

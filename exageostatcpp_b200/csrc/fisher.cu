@@ -20,10 +20,11 @@
 // The reference differentiates K_nu in nu by a forward difference with step
 // 1e-9 (src/helpers/BasselFunction.cpp:23-33); here F_nu(x) = x^nu K_nu(x) itself is
 // differentiated: the last two terms are dF/dnu, from the six-point central
-// difference with step h = 2e-3 (truncation h^6 / 140 d^7F/dnu^7), and dC/dbeta = sigma2 c (F_nu+1 - 2 nu F_nu) / beta.  F comes from the Chebyshev
-// tables of the generator (e^x F, one table per nu value), where the direct
-// series and continued fraction cost thousands of operations for every order
-// (N = 1,600: derivatives 2.7 ms of direct evaluations, 0.1 from the tables).
+// difference with step h = 2e-3 (truncation h^6 / 140 d^7F/dnu^7), and
+// dC/dbeta = sigma2 c (F_nu+1 - 2 nu F_nu) / beta.  F comes from the generator's
+// tables (e^x F, one per order), where the direct series and continued fraction
+// cost thousands of operations for every order (N = 1,600: derivatives 2.7 ms of
+// direct evaluations, 0.1 from the tables).
 #include <cmath>
 #include <memory>
 #include <vector>
@@ -41,12 +42,12 @@ struct FisherParams {
 // Orders whose F the derivatives need: nu, nu + 1, nu +- h, nu +- 2 h, nu +- 3 h.
 constexpr int kFisherOrders = 8;
 constexpr double kFisherStep = 2e-3;
-constexpr int kFisherTabBytes = kFisherOrders * kKtabDoubles * (int)sizeof(double);
+constexpr int kFisherTabBytes = kFisherOrders * kKtabShared * (int)sizeof(double);
 
 // F_nu(x) = x^nu K_nu(x) of the order of p (kind 2), from its table where x lies in it.
 __device__ __forceinline__ double bessel_f(double x, bool in_table, int idx, double t, double ex,
                                            const MaternParams& p, const double* __restrict__ tab) {
-  if (in_table && p.table) return ktab_sum(tab + idx * kKtabStride, t) * ex;
+  if (in_table && p.table) return ktab_sum(tab + idx * kKtabRow, t) * ex;
   bool scaled;
   const double k = bessel_k_general(x, p, scaled);
   return pow(x, p.nu) * (scaled ? k * ex : k);
@@ -58,8 +59,9 @@ __global__ void __launch_bounds__(256)
 matern_derivatives_kernel(const double* __restrict__ x, const double* __restrict__ y, int n, int np,
                           FisherParams q, const MaternParams* __restrict__ orders, const double* __restrict__ tabs,
                           double* __restrict__ d) {
-  extern __shared__ double stab[];  // kFisherTabBytes
-  for (int i = threadIdx.x; i < kFisherOrders * kKtabDoubles; i += 256) stab[i] = tabs[i];
+  extern __shared__ __align__(16) double stab[];  // kFisherTabBytes
+  for (int i = threadIdx.x; i < kFisherOrders * kKtabDoubles; i += 256)
+    stab[(i / kKtabStride) * kKtabRow + i % kKtabStride] = tabs[i];
   __syncthreads();
   const long long nn = (long long)np * np;
   for (long long idx = (long long)blockIdx.x * 256 + threadIdx.x; idx < nn; idx += (long long)gridDim.x * 256) {
@@ -77,7 +79,7 @@ matern_derivatives_kernel(const double* __restrict__ x, const double* __restrict
         double f[kFisherOrders];
 #pragma unroll
         for (int o = 0; o < kFisherOrders; ++o)
-          f[o] = bessel_f(e, in_table, at, t, ex, orders[o], stab + o * kKtabDoubles);
+          f[o] = bessel_f(e, in_table, at, t, ex, orders[o], stab + o * kKtabShared);
         const double df = (45.0 * (f[2] - f[3]) - 9.0 * (f[4] - f[5]) + (f[6] - f[7])) / (60.0 * kFisherStep);
         ds = q.con * f[0];
         db = q.sigma2 * q.con / q.beta * (f[1] - 2.0 * q.nu * f[0]);

@@ -19,6 +19,10 @@ int launch_matern_tiles(double* tiles, const double* x, const double* y, int n, 
 void launch_matern_ktab(const MaternParams* params, double* tab, int nproblems, cudaStream_t st);
 int launch_matern_block(double* a, int lda, int rows, int cols, const double* x1, const double* y1,
                         const double* x2, const double* y2, const MaternParams& p, cudaStream_t st);
+// The same with theta's parameters and table already on the device (launch_matern_ktab).
+int launch_matern_block_tab(double* a, int lda, int rows, int cols, const double* x1, const double* y1,
+                            const double* x2, const double* y2, const MaternParams* params, const double* ktab,
+                            cudaStream_t st);
 
 // Factorisation building blocks (potrf.cu).  All offsets are element offsets
 // inside a tile; tiles are addressed by lower-tile slot.

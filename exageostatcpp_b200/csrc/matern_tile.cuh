@@ -9,12 +9,14 @@ constexpr int kGenThreads = 256;
 constexpr int kGenPairsPerThread = 8;
 constexpr int kGenPairsPerBlock = kGenThreads * kGenPairsPerThread;  // 4096 elements per block
 
-// Copies one problem's Chebyshev table into shared memory when its nu uses it.
+// Copies one problem's table into shared memory (kKtabShared doubles, 16-byte
+// aligned) when its nu uses it.
 // Every thread of the block calls it (it ends with a barrier).
 __device__ __forceinline__ void stage_ktab(double* __restrict__ stab, const double* __restrict__ tab,
                                            const MaternParams& p) {
   if (p.table) {
-    for (int i = threadIdx.x; i < kKtabDoubles; i += blockDim.x) stab[i] = tab[i];
+    for (int i = threadIdx.x; i < kKtabDoubles; i += blockDim.x)
+      stab[(i / kKtabStride) * kKtabRow + i % kKtabStride] = tab[i];
   }
   __syncthreads();
 }
@@ -30,14 +32,13 @@ __device__ __forceinline__ void matern_tile_pairs(Out* __restrict__ tile, const 
                                                   const double* __restrict__ y, int n, int ts, int ti, int tj,
                                                   long long pair0, const MaternParams& p,
                                                   const double* __restrict__ tab) {
-  const long long pairs_per_tile = (long long)ts * ts / 2;
+  const double rbeta = 1.0 / p.beta;
+  const long long e0 = 2 * (pair0 + threadIdx.x);
+  int c = (int)(e0 / ts), r = (int)(e0 - (long long)c * ts);
+  // the next pair of this thread is 2 * kGenThreads elements on
+  const int dc = 2 * kGenThreads / ts, dr = 2 * kGenThreads - dc * ts;
 #pragma unroll 1
-  for (int i = 0; i < kGenPairsPerThread; ++i) {
-    const long long pair = pair0 + i * kGenThreads + threadIdx.x;
-    if (pair >= pairs_per_tile) return;
-    const long long e = pair * 2;
-    const int c = (int)(e / ts);
-    const int r = (int)(e - (long long)c * ts);
+  for (int i = 0; i < kGenPairsPerThread && c < ts; ++i) {
     const int gr = ti * ts + r;
     const int gc = tj * ts + c;
     double v0, v1;
@@ -48,13 +49,20 @@ __device__ __forceinline__ void matern_tile_pairs(Out* __restrict__ tile, const 
       const double xc = x[gc], yc = y[gc];
       const double2 xr = *reinterpret_cast<const double2*>(x + gr);
       const double2 yr = *reinterpret_cast<const double2*>(y + gr);
-      v0 = (gr < n) ? matern_from_dist_tab(euclid_dist(xr.x, yr.x, xc, yc), p, tab) : 0.0;
-      v1 = (gr + 1 < n) ? matern_from_dist_tab(euclid_dist(xr.y, yr.y, xc, yc), p, tab) : 0.0;
+      v0 = (gr < n) ? matern_from_dist_tab(euclid_dist(xr.x, yr.x, xc, yc), p, rbeta, tab) : 0.0;
+      v1 = (gr + 1 < n) ? matern_from_dist_tab(euclid_dist(xr.y, yr.y, xc, yc), p, rbeta, tab) : 0.0;
     }
+    const long long e = (long long)c * ts + r;
     if constexpr (sizeof(Out) == 8) {
       *reinterpret_cast<double2*>(tile + e) = make_double2(v0, v1);
     } else {
       *reinterpret_cast<float2*>(tile + e) = make_float2((float)v0, (float)v1);
+    }
+    c += dc;
+    r += dr;
+    if (r >= ts) {
+      r -= ts;
+      ++c;
     }
   }
 }

@@ -39,7 +39,7 @@ __global__ void __launch_bounds__(kGenThreads)
 matern_mixed_kernel(double* __restrict__ band, float* __restrict__ off, const double* __restrict__ x,
                     const double* __restrict__ y, int n, int ts, const int4* __restrict__ tinfo, long long t0,
                     const MaternParams* __restrict__ pp, const double* __restrict__ ktab) {
-  __shared__ double stab[kKtabDoubles];
+  __shared__ __align__(16) double stab[kKtabShared];
   const MaternParams p = *pp;
   stage_ktab(stab, ktab, p);
   const int4 ti = tinfo[t0 + blockIdx.y];
@@ -347,6 +347,7 @@ void launch_mixed_solve(const double* band, const float* off, const double* inv,
 // ---------------------------------------------------------------------------
 constexpr int kResBlk = 256;    // rows (and columns) per block = threads per CTA
 constexpr int kResSuper = 8;    // most blocks per super-block side
+constexpr int kResSmemBytes = (kKtabShared + kResBlk / 32 * kResBlk) * (int)sizeof(double);  // tables, warp sums
 
 __host__ __device__ __forceinline__ int res_blocks(int n) { return (n + kResBlk - 1) / kResBlk; }
 // Blocks per super-block side: as many as keep at least ~24 super-blocks per
@@ -362,12 +363,14 @@ matern_residual_partial_kernel(const double* __restrict__ x, const double* __res
                                const double* __restrict__ v, int n, const MaternParams* __restrict__ pp,
                                const double* __restrict__ ktab, double* __restrict__ rowpart,
                                double* __restrict__ colpart) {
-  __shared__ double stab[kKtabDoubles];
+  extern __shared__ __align__(16) double res_smem[];  // kResSmemBytes
+  double* stab = res_smem;
+  double(*red)[kResBlk] = reinterpret_cast<double(*)[kResBlk]>(res_smem + kKtabShared);
   __shared__ double xs[kResBlk], ys[kResBlk], vs[kResBlk];
-  __shared__ double red[kResBlk / 32][kResBlk];
   __shared__ double colacc[kResSuper][kResBlk];  // column sums of each column block (thread = column)
   const MaternParams p = *pp;
   stage_ktab(stab, ktab, p);
+  const double rbeta = 1.0 / p.beta;
   // super-block (sbi, sbj), sbj <= sbi, from the linear index
   const int L = blockIdx.x;
   int sbi = (int)((sqrt(8.0 * (double)L + 1.0) - 1.0) * 0.5);
@@ -401,15 +404,35 @@ matern_residual_partial_kernel(const double* __restrict__ x, const double* __res
       __syncthreads();
       const bool diag = (bj == bi);
       const int m = min(kResBlk, n - jb);
-      for (int jj = 0; jj < m; ++jj) {
-        double c = 0.0;
-        if (row && (!diag || jj <= t)) c = matern_from_dist_tab(euclid_dist(xi, yi, xs[jj], ys[jj]), p, stab);
-        racc = fma(c, vs[jj], racc);
-        // column jj gets C(i, jj) v_i from every row i below it (i > j)
-        double cc = (!diag || jj < t) ? c * vi : 0.0;
+      // eight columns at a time: C(i, j) v_j into the row sum, and the columns'
+      // C(i, j) v_i (from every row i below column j) summed over the warp by
+      // halving exchanges: 9 shuffles for 8 columns instead of 40
+      for (int j0 = 0; j0 < m; j0 += 8) {
+        double cc[8];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) cc += __shfl_xor_sync(0xffffffffu, cc, o);
-        if (lane == 0) red[warp][jj] = cc;
+        for (int q8 = 0; q8 < 8; ++q8) {
+          const int jj = j0 + q8;  // columns past m read zeroed locations and add nothing
+          double c = 0.0;
+          if (row && jj < m && (!diag || jj <= t))
+            c = matern_from_dist_tab(euclid_dist(xi, yi, xs[jj], ys[jj]), p, rbeta, stab);
+          racc = fma(c, vs[jj], racc);
+          cc[q8] = (!diag || jj < t) ? c * vi : 0.0;
+        }
+#pragma unroll
+        for (int h = 4; h >= 1; h >>= 1) {
+          const int bit = 4 * h;  // lanes with this bit keep the upper half of the columns
+          const bool up = lane & bit;
+#pragma unroll
+          for (int q8 = 0; q8 < 4; ++q8)
+            if (q8 < h) {
+              const double send = up ? cc[q8] : cc[q8 + h];
+              const double keep = up ? cc[q8 + h] : cc[q8];
+              cc[q8] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
+            }
+        }
+        cc[0] += __shfl_xor_sync(0xffffffffu, cc[0], 2);
+        cc[0] += __shfl_xor_sync(0xffffffffu, cc[0], 1);
+        if ((lane & 3) == 0) red[warp][j0 + (lane >> 2)] = cc[0];
       }
       __syncthreads();
       double sum = 0.0;
@@ -452,7 +475,11 @@ void launch_matern_residual(const double* x, const double* y, const double* z, c
   double* rowpart = scratch;
   double* colpart = scratch + (long long)ns * n;
   const unsigned grid = (unsigned)((long long)ns * (ns + 1) / 2);
-  matern_residual_partial_kernel<<<grid, kResBlk, 0, st>>>(x, y, v, n, params, ktab, rowpart, colpart);
+  static std::once_flag attr[64];
+  once_per_device(attr, []() {
+    cudaFuncSetAttribute(matern_residual_partial_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kResSmemBytes);
+  });
+  matern_residual_partial_kernel<<<grid, kResBlk, kResSmemBytes, st>>>(x, y, v, n, params, ktab, rowpart, colpart);
   residual_reduce_kernel<<<(np + 255) / 256, 256, 0, st>>>(z, rowpart, colpart, n, np, r);
 }
 
