@@ -216,12 +216,20 @@ gemv_mixed_kernel(const double* __restrict__ band, const float* __restrict__ off
   }
 }
 
-// z_i -= L_ki^T z_k for every tile column i < k; one warp per column of tile (k, i).
+// z_i -= L_ki^T z_k for every tile column i < k; one warp per column of tile (k, i),
+// 16 bytes per lane and load.
 template <typename Tile>
 __device__ __forceinline__ double col_dot(const Tile* __restrict__ col, const double* __restrict__ zk, int ts,
                                           int lane) {
+  constexpr int VEC = 16 / (int)sizeof(Tile);
   double acc = 0.0;
-  for (int r = lane; r < ts; r += 32) acc = fma((double)col[r], zk[r], acc);
+#pragma unroll 4
+  for (int r = lane * VEC; r < ts; r += 32 * VEC) {
+    double v[VEC];
+    load_vec(col + r, v);
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) acc = fma(v[i], zk[r + i], acc);
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
   return acc;
@@ -253,44 +261,48 @@ inv_apply_t_kernel(const double* __restrict__ X, int ts, const double* __restric
   if (i >= ts) return;
   const double* col = X + (long long)i * ts;
   double acc = 0.0;
-  for (int j = lane; j <= i; j += 32) acc = fma(col[j], in[j], acc);
+#pragma unroll 4
+  for (int j = 2 * lane; j <= i; j += 64) {
+    const double2 v = *reinterpret_cast<const double2*>(col + j);
+    acc = fma(v.x, in[j], acc);
+    if (j + 1 <= i) acc = fma(v.y, in[j + 1], acc);
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
   if (lane == 0) out[i] = acc;
 }
 
-// out = L_kk^-T in = X in: out[i] = sum_{j >= i} X[i, j] in[j]; 64 rows x 4
-// column groups per block, fixed reduction order.  Dynamic shared memory: ts doubles.
+// out = L_kk^-T in = X in: out[i] = sum_{j >= i} X[i, j] in[j]; 16 rows x 32
+// column groups per block (a group reads 128 bytes of a column, 16 bytes a
+// thread), fixed reduction order.  Latency-bound: 64 rows a block left 16 blocks
+// at ts = 1,024 (43 us a launch, 22 with 64 blocks).  Dynamic shared memory: ts
+// doubles.
+constexpr int kInvRows = 16;
 __global__ void __launch_bounds__(256)
 inv_apply_kernel(const double* __restrict__ X, int ts, const double* __restrict__ in, double* __restrict__ out) {
   extern __shared__ double ins[];
-  __shared__ double red[4][kNB];
+  __shared__ double red[32][kInvRows + 1];
   for (int c = threadIdx.x; c < ts; c += blockDim.x) ins[c] = in[c];
   __syncthreads();
-  const int rl = threadIdx.x & (kNB - 1), g = threadIdx.x / kNB;
-  const int i = blockIdx.x * kNB + rl;
-  // four interleaved sums per thread keep sixteen loads in flight; the column
-  // order within each sum and the final combination are fixed
-  double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-  if (i < ts) {
-    const double* xr = X + i;
-    int j = blockIdx.x * kNB + g;
-    for (; j + 12 < ts; j += 16) {
-      const double x0 = (j >= i) ? xr[(long long)j * ts] : 0.0;
-      const double x1 = (j + 4 >= i) ? xr[(long long)(j + 4) * ts] : 0.0;
-      const double x2 = (j + 8 >= i) ? xr[(long long)(j + 8) * ts] : 0.0;
-      const double x3 = (j + 12 >= i) ? xr[(long long)(j + 12) * ts] : 0.0;
-      a0 = fma(x0, ins[j], a0);
-      a1 = fma(x1, ins[j + 4], a1);
-      a2 = fma(x2, ins[j + 8], a2);
-      a3 = fma(x3, ins[j + 12], a3);
-    }
-    for (; j < ts; j += 4)
-      if (j >= i) a0 = fma(xr[(long long)j * ts], ins[j], a0);
+  const int rl = 2 * (threadIdx.x & 7), g = threadIdx.x >> 3;
+  const int i0 = blockIdx.x * kInvRows, i = i0 + rl;
+  double a0 = 0.0, a1 = 0.0;
+  const double* xr = X + i;
+#pragma unroll 8
+  for (int j = i0 + g; j < ts; j += 32) {
+    const double2 v = *reinterpret_cast<const double2*>(xr + (long long)j * ts);
+    if (j >= i) a0 = fma(v.x, ins[j], a0);
+    if (j >= i + 1) a1 = fma(v.y, ins[j], a1);
   }
-  red[g][rl] = (a0 + a1) + (a2 + a3);
+  red[g][rl] = a0;
+  red[g][rl + 1] = a1;
   __syncthreads();
-  if (g == 0 && i < ts) out[i] = ((red[0][rl] + red[1][rl]) + red[2][rl]) + red[3][rl];
+  if (threadIdx.x < kInvRows) {
+    double s = red[0][threadIdx.x];
+#pragma unroll
+    for (int q = 1; q < 32; ++q) s += red[q][threadIdx.x];
+    out[i0 + threadIdx.x] = s;
+  }
 }
 
 __global__ void add_inplace_kernel(double* __restrict__ a, const double* __restrict__ b, int n) {
@@ -322,7 +334,7 @@ void launch_mixed_solve(const double* band, const float* off, const double* inv,
     *launches += 2;
   }
   for (int k = nt - 1; k >= 0; --k) {
-    inv_apply_kernel<<<(ts + kNB - 1) / kNB, 256, ts * sizeof(double), st>>>(inv + k * ts2, ts, v + (long long)k * ts,
+    inv_apply_kernel<<<ts / kInvRows, 256, ts * sizeof(double), st>>>(inv + k * ts2, ts, v + (long long)k * ts,
                                                                                tmp);
     if (k > 0) {
       gemv_t_mixed_kernel<<<dim3((ts + 7) / 8, k), 256, 0, st>>>(band, off, ts, nt, b, k, tmp, v);
