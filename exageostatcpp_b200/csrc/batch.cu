@@ -57,7 +57,7 @@ matern_batch_kernel(double* __restrict__ tiles, const double* __restrict__ x, co
 // problem with more than k tile rows, and the flush of the previous step (pk,
 // pkb, pnb) of every problem that had one: blocks x < steps are row chunks, the
 // rest scratch chunks; block y is the problem.
-__global__ void __launch_bounds__(kStepThreads, 512 / kStepThreads)
+__global__ void __launch_bounds__(kStepThreads, 2)
 panel_step_batch_kernel(double* tiles, int ts, int k, int kb, int nb, int steps, int active, int pk, int pkb, int pnb,
                         int pactive, int parity, const long long* __restrict__ tile_base, const int* __restrict__ ntv,
                         int* info, double* z, const long long* __restrict__ loc_base, double* __restrict__ scratch) {

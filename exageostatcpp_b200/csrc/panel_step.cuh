@@ -9,12 +9,14 @@
 // rows its update needs, so no CTA waits for another one.  It is bound by the
 // chain of 64 dependent pivots, not by work: three dependent launches for the
 // three parts took 58-70 us per step whatever the panel's height, a step now
-// takes about 18 us (N = 1,600, tile 320: panels 1.46 -> 0.68 ms per evaluation, the
-// forward solve below 0.51 -> 0; N = 10,000, tile 960: 11.5 -> 6.4 and 6.9 -> 0).
+// takes about 13 us (N = 1,600, tile 320: panels 1.46 -> 0.44 ms per evaluation, the
+// forward solve below 0.51 -> 0; N = 10,000, tile 960: 11.5 -> 5.0 and 6.9 -> 0).
 // The redundant arithmetic runs on SMs that would otherwise be idle.
 // Outer blocks are two 64-column blocks wide: wider ones make every CTA solve
 // more foreign chunks (each costs as much FP64 time as its own), narrower ones
-// leave more to the K = 64 update launches.
+// leave more to the K = 64 update launches (N = 1,600 / N = 20,011 mixed / 512-problem
+// batch: one block 533 us / 32.6 ms / 83.7 ms, two 556 / 31.7 / 78.3, three 583 /
+// 32.0 / 86.0).
 //
 // The pivots run in one warp, eight at a time in registers: every lane holds
 // the 8 x 8 block, so no pivot waits for an exchange between lanes (16 columns
@@ -43,11 +45,8 @@ namespace egs {
 constexpr int kStep = 64;           // columns of a step, rows of a chunk
 constexpr int kStepLd = 68;         // shared-memory column stride: fragment loads hit distinct banks
 constexpr int kStepBlock = kStep * kStepLd;
-#ifndef EGS_STEP_BLOCKS
-#define EGS_STEP_BLOCKS 2
-#endif
-constexpr int kStepMaxBlocks = EGS_STEP_BLOCKS;   // most 64-column blocks of an outer block
-constexpr int kStepThreads = 64 * kStepMaxBlocks + 128;
+constexpr int kStepMaxBlocks = 2;   // most 64-column blocks of an outer block
+constexpr int kStepThreads = 128 * ((2 * kStepMaxBlocks + 4) / 3);
 constexpr int kStepHelpers = 3 * kStepThreads / 128;  // warps beside the pivot warp's sub-partition
 static_assert(2 * kStepMaxBlocks + 2 <= kStepHelpers, "two warps per row chunk and two for the diagonal block");
 constexpr int kScratchLd = kStepMaxBlocks * kStep;
@@ -142,26 +141,26 @@ __device__ __forceinline__ double step_rsqrt(double d) {
 
 // Cholesky of the 8 x 8 lower block l in registers, every lane the same values:
 // no exchange between lanes, so the chain per pivot is rsqrt, scale and one
-// fused multiply-add.  iv[j] = 1 / L_jj.  Returns a mask of the pivots outside
+// fused multiply-add.  l[j][j] becomes 1 / L_jj.  Returns a mask of the pivots outside
 // the range of the fast rsqrt (zero, negative, NaN, subnormal, huge); kSafe uses
 // rsqrt() and returns the mask of pivots that are not positive (or NaN).
 template <bool kSafe>
-__device__ __forceinline__ unsigned step_factor8(double (&l)[8][8], double (&iv)[8]) {
+__device__ __forceinline__ unsigned step_factor8(double (&l)[8][8]) {
   unsigned mask = 0;
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     const double d = l[j][j];
     if constexpr (kSafe) {
       if (!(d > 0.0)) mask |= 1u << j;
-      iv[j] = rsqrt(d);
+      l[j][j] = rsqrt(d);
     } else {
       // exponent field in [0x05d, 0x79d): about 1e-280 .. 1e+280, sign bit clear
       if ((unsigned)__double2hiint(d) - 0x05d00000u >= 0x74000000u) mask |= 1u << j;
-      iv[j] = step_rsqrt(d);
+      l[j][j] = step_rsqrt(d);
     }
 #pragma unroll
     for (int i = 0; i < 8; ++i)
-      if (i > j) l[i][j] *= iv[j];
+      if (i > j) l[i][j] *= l[j][j];
 #pragma unroll
     for (int c = 0; c < 8; ++c)
 #pragma unroll
@@ -171,11 +170,11 @@ __device__ __forceinline__ unsigned step_factor8(double (&l)[8][8], double (&iv)
   return mask;
 }
 
-// y := y L^-T for one row of 8 values.
-__device__ __forceinline__ void step_subst8(double (&y)[8], const double (&l)[8][8], const double (&iv)[8]) {
+// y := y L^-T for one row of 8 values (l[j][j] = 1 / L_jj).
+__device__ __forceinline__ void step_subst8(double (&y)[8], const double (&l)[8][8]) {
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
-    y[j] *= iv[j];
+    y[j] *= l[j][j];
 #pragma unroll
     for (int c = 0; c < 8; ++c)
       if (c > j) y[c] = fma(-y[j], l[c][j], y[c]);
@@ -220,7 +219,7 @@ __device__ __forceinline__ void step_pivots8(double* D, double* pinv, int b, int
     step_store8(col + hi + lane, y);
     __syncwarp();
   }
-  double l[8][8], iv[8];
+  double l[8][8];
   auto load_block = [&]() {
 #pragma unroll
     for (int c = 0; c < 8; ++c)
@@ -233,18 +232,18 @@ __device__ __forceinline__ void step_pivots8(double* D, double* pinv, int b, int
         }
   };
   load_block();
-  if (step_factor8<false>(l, iv)) {
+  if (step_factor8<false>(l)) {
     load_block();
-    const unsigned bad = step_factor8<true>(l, iv);
+    const unsigned bad = step_factor8<true>(l);
     if (bad && info && lane == 0) atomicCAS(info, 0, gcol + 8 * b + __ffs(bad));
   }
   step_load8(y, col + hi + lane);  // not kept across the pivots: registers are short
-  step_subst8(y, l, iv);
+  step_subst8(y, l);
   __syncwarp();
   step_store8(col + hi + lane, y);
   if (lane == 0) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) pinv[8 * b + j] = iv[j];
+    for (int j = 0; j < 8; ++j) pinv[8 * b + j] = l[j][j];
   }
   if (b < 4) {
     // the other half against L and 1 / L_jj in shared memory (registers are short)
@@ -376,18 +375,24 @@ __device__ __forceinline__ void panel_step_body(double* __restrict__ sm, double*
     cp_async16(D + c * kStepLd + r, col + (long long)(kb + c) * ts + kb + r);
   }
   cp_async_commit();
-  for (int b = 0; b < nrc; ++b) {
-    const double* src = (b == 0) ? own : col + kb + kStep * b;
-    double* dst = A + b * kStepBlock;
-    for (int e = tid; e < kStep * kStep / 2; e += kStepThreads) {
-      const int c = e >> 5, r = 2 * (e & 31);
-      cp_async16(dst + c * kStepLd + r, src + (long long)(kb + c) * ts + r);
-    }
-  }
-  cp_async_commit();
   if (z && tid < kStep) zk[tid] = z[kb + tid];
-  cp_async_wait<1>();
+  // the rows' part of z, subtracted from at the end by the last two warps
+  const int zr = tid - (kStepThreads - kStep);
+  const double zi = (z && chunk >= 0 && zr >= 0) ? z[g + zr] : 0.0;
+  cp_async_wait<0>();
   __syncthreads();
+  // the pivots start; the row blocks, needed two rounds later, arrive beside them
+  if (warp != 0) {
+    for (int b = 0; b < nrc; ++b) {
+      const double* src = (b == 0) ? own : col + kb + kStep * b;
+      double* dst = A + b * kStepBlock;
+      for (int e = tid - 32; e < kStep * kStep / 2; e += kStepThreads - 32) {
+        const int c = e >> 5, r = 2 * (e & 31);
+        cp_async16(dst + c * kStepLd + r, src + (long long)(kb + c) * ts + r);
+      }
+    }
+    cp_async_commit();
+  }
 
   // Warp 0 runs the pivots and has its SM sub-partition to itself (an FP64 MMA
   // of another warp would hold up its chain); warps 1-3 (mod 4) are helpers:
@@ -482,17 +487,16 @@ __device__ __forceinline__ void panel_step_body(double* __restrict__ sm, double*
     }
     if (z && tid < kStep) out[kScratchLd * kStep + tid] = zk[tid];
   }
-  if (z && chunk >= 0 && warp >= kStepThreads / 32 - 2) {
-    const int r = tid - (kStepThreads - kStep);
+  if (z && chunk >= 0 && zr >= 0) {
     double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
 #pragma unroll 4
     for (int c = 0; c < kStep; c += 4) {
-      s0 = fma(A[c * kStepLd + r], zk[c], s0);
-      s1 = fma(A[(c + 1) * kStepLd + r], zk[c + 1], s1);
-      s2 = fma(A[(c + 2) * kStepLd + r], zk[c + 2], s2);
-      s3 = fma(A[(c + 3) * kStepLd + r], zk[c + 3], s3);
+      s0 = fma(A[c * kStepLd + zr], zk[c], s0);
+      s1 = fma(A[(c + 1) * kStepLd + zr], zk[c + 1], s1);
+      s2 = fma(A[(c + 2) * kStepLd + zr], zk[c + 2], s2);
+      s3 = fma(A[(c + 3) * kStepLd + zr], zk[c + 3], s3);
     }
-    z[g + r] -= (s0 + s1) + (s2 + s3);
+    z[g + zr] = zi - ((s0 + s1) + (s2 + s3));
   }
   // update of the later columns of the outer block: 16 x 32 warp tiles, K = 64
 #pragma unroll 1

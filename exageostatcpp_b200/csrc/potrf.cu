@@ -22,8 +22,12 @@ namespace egs {
 
 // One 64-column step of a panel (panel_step_body), and the flush of the step
 // before it: blocks [0, steps) are the step's row chunks, the others copy the
-// scratch slot of the previous step to its place.
-__global__ void __launch_bounds__(kStepThreads, 512 / kStepThreads)
+// scratch slot of the previous step to its place.  CTAS per SM: one leaves the
+// pivot warp enough registers (two cap them at 128 and spill: N = 1,600, 25 chunks,
+// 570 -> 550 us per evaluation with one); two are faster once the chunks fill the
+// SMs more than once (N = 40,000, up to 624: 665 -> 663 ms with two).
+template <int CTAS>
+__global__ void __launch_bounds__(kStepThreads, CTAS)
 panel_step_kernel(double* col, int ts, int nchunk, int kb, int nb, int gcol, int* info, double* z,
                   double* __restrict__ out, const double* __restrict__ pslot, double* pcol, int pkb, double* pz) {
   extern __shared__ __align__(16) double step_smem[];
@@ -63,15 +67,17 @@ int launch_panel_step(double* col, int ts, int rows_below, int kb, int nb, int g
                       PanelChain& ch, cudaStream_t st) {
   static std::once_flag done[64];
   once_per_device(done, []() {
-    cudaFuncSetAttribute(panel_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         panel_step_smem(kStepMaxBlocks - 1));
+    constexpr auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaFuncSetAttribute(panel_step_kernel<1>, attr, panel_step_smem(kStepMaxBlocks - 1));
+    cudaFuncSetAttribute(panel_step_kernel<2>, attr, panel_step_smem(kStepMaxBlocks - 1));
   });
   const int nchunk = rows_below / kStep;
   double* out = ch.scratch + (long long)ch.parity * kScratchSlot;
   const double* pslot = ch.scratch + (long long)(ch.parity ^ 1) * kScratchSlot;
   const int grid = (nchunk > 0 ? nchunk : 1) + ch.chunks;
-  panel_step_kernel<<<grid, kStepThreads, panel_step_smem(nb), st>>>(col, ts, nchunk, kb, nb, gcol, info, z, out,
-                                                                     pslot, ch.col, ch.kb, ch.z);
+  auto kern = nchunk > gemm_num_sms() ? panel_step_kernel<2> : panel_step_kernel<1>;
+  kern<<<grid, kStepThreads, panel_step_smem(nb), st>>>(col, ts, nchunk, kb, nb, gcol, info, z, out, pslot, ch.col,
+                                                        ch.kb, ch.z);
   ch.col = col;
   ch.kb = kb;
   ch.chunks = 1 + (nb < nchunk ? nb : nchunk);
