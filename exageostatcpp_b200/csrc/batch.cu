@@ -53,29 +53,37 @@ matern_batch_kernel(double* __restrict__ tiles, const double* __restrict__ x, co
                     (long long)blockIdx.x * kGenPairsPerBlock, prm, stab);
 }
 
+// 64-row chunks below the block at column kb of tile column k of a problem of n
+// points (factor_rows); negative when the block lies beyond the problem's rows.
+__host__ __device__ inline int batch_chunks(int n, int ts, int k, int kb) {
+  return (factor_rows(n) - k * ts - kb) / kStep - 1;
+}
+
 // One 64-column panel step (tile column k, column kb, panel_step_body) of every
-// problem with more than k tile rows, and the flush of the previous step (pk,
-// pkb, pnb) of every problem that had one: blocks x < steps are row chunks, the
-// rest scratch chunks; block y is the problem.
+// problem whose rows reach it, and the flush of the previous step (pk, pkb) of
+// every problem that had one: blocks x < steps are row chunks, the rest scratch
+// chunks; block y is the problem.
 __global__ void __launch_bounds__(kStepThreads, 2)
-panel_step_batch_kernel(double* tiles, int ts, int k, int kb, int nb, int steps, int active, int pk, int pkb, int pnb,
-                        int pactive, int parity, const long long* __restrict__ tile_base, const int* __restrict__ ntv,
-                        int* info, double* z, const long long* __restrict__ loc_base, double* __restrict__ scratch) {
+panel_step_batch_kernel(double* tiles, int ts, int k, int kb, int steps, int active, int pk, int pkb, int pactive,
+                        int parity, const long long* __restrict__ tile_base, const int* __restrict__ ntv,
+                        const int* __restrict__ nvec, int* info, double* z, const long long* __restrict__ loc_base,
+                        double* __restrict__ scratch) {
   extern __shared__ __align__(16) double step_smem[];
-  const int p = blockIdx.y, nt = ntv[p];
+  const int p = blockIdx.y, nt = ntv[p], n = nvec[p];
   double* slots = scratch + (long long)p * kScratchDoubles;
   double* pool = tiles + tile_base[p] * (long long)ts * ts;
   if ((int)blockIdx.x < steps) {
     if (p >= active) return;
-    const int nchunk = ((nt - k) * ts - kb) / kStep - 1;
-    if ((int)blockIdx.x >= (nchunk > 0 ? nchunk : 1)) return;
+    const int nchunk = batch_chunks(n, ts, k, kb);
+    if (nchunk < 0 || (int)blockIdx.x >= max(1, nchunk)) return;
     panel_step_body(step_smem, pool + tile_slot(k, k, nt) * (long long)ts * ts, ts, nchunk > 0 ? (int)blockIdx.x : -1,
-                    kb, nb, k * ts + kb, blockIdx.x == 0 ? info + p : nullptr, z + loc_base[p] + (long long)k * ts,
+                    kb, panel_outer_rest(min(ts, factor_rows(n) - k * ts), kb), k * ts + kb,
+                    blockIdx.x == 0 ? info + p : nullptr, z + loc_base[p] + (long long)k * ts,
                     slots + parity * kScratchSlot);
   } else {
     const int f = blockIdx.x - steps;
-    const int nchunk = p < pactive ? ((nt - pk) * ts - pkb) / kStep - 1 : -1;
-    if (nchunk < 0 || f > min(pnb, nchunk)) return;
+    const int nchunk = p < pactive ? batch_chunks(n, ts, pk, pkb) : -1;
+    if (nchunk < 0 || f > min(panel_outer_rest(min(ts, factor_rows(n) - pk * ts), pkb), nchunk)) return;
     panel_flush_body(slots + (parity ^ 1) * kScratchSlot, pool + tile_slot(pk, pk, nt) * (long long)ts * ts, ts, pkb,
                      f, z + loc_base[p] + (long long)pk * ts);
   }
@@ -232,13 +240,13 @@ int build_jobs(egs_batch* b) {
     const int A1 = (k + 1 < b->nt_max) ? b->active[k + 1] : 0;
     int KB = 0;  // first column of the current outer block
     for (int kb = 0; kb < ts; kb += kBatchInner) {
-      if (panel_outer_blocks(ts, kb) > 1) continue;
+      if (panel_outer_rest(ts, kb) > 0) continue;
       const int KE = kb + kBatchInner;
       std::vector<GemmDesc> js;
-      if (KE < ts) {
-        const int r0 = k * ts + KE;
-        for (int p = 0; p < A; ++p)
-          js.push_back(job_desc(b, p, b->nt[p] * ts - r0, ts - KE, KE - KB, r0, KB, k, r0, KB, k, r0, r0, 1));
+      const int r0 = k * ts + KE;
+      for (int p = 0; p < A && KE < ts; ++p) {
+        const int below = factor_rows(b->n[p]) - r0, right = std::min(ts, factor_rows(b->n[p]) - k * ts) - KE;
+        if (right > 0) js.push_back(job_desc(b, p, below, right, KE - KB, r0, KB, k, r0, KB, k, r0, r0, 1));
       }
       add_launch(b->panel_launch, js);
       KB = KE;
@@ -246,7 +254,7 @@ int build_jobs(egs_batch* b) {
     std::vector<GemmDesc> js;
     for (int p = 0; p < A1; ++p) {
       const int r0 = (k + 1) * ts;
-      const int m = b->nt[p] * ts - r0;
+      const int m = factor_rows(b->n[p]) - r0;
       js.push_back(job_desc(b, p, m, m, ts, r0, 0, k, r0, 0, k, r0, r0, 1));
     }
     add_launch(b->trail_launch, js);
@@ -291,22 +299,25 @@ int enqueue_batch_eval(egs_batch* b) {
                          panel_step_smem(kStepMaxBlocks - 1));
   });
   int li = 0, parity = 0;
-  int pk = 0, pkb = 0, pnb = 0, pactive = 0;  // the step still in its scratch slot
+  int pk = 0, pkb = 0, pactive = 0;  // the step still in its scratch slot
+  const int n_max = *std::max_element(b->n.begin(), b->n.end());
   for (int k = 0; k < b->nt_max; ++k) {
     const int A = b->active[k];
     for (int kb = 0; kb < ts; kb += kBatchInner) {
-      const int nb = panel_outer_blocks(ts, kb) - 1;
-      const int steps = std::max(1, ((b->nt_max - k) * ts - kb) / kStep - 1);
-      panel_step_batch_kernel<<<dim3(steps + (pactive ? 1 + pnb : 0), std::max(A, pactive)), kStepThreads,
-                                panel_step_smem(nb), st>>>(b->tiles, ts, k, kb, nb, steps, A, pk, pkb, pnb, pactive,
-                                                           parity, b->d_tile_base, b->d_nt, b->info, b->z,
-                                                           b->d_loc_base, b->scratch);
-      ++b->launches_per_eval;
-      pk = k;
-      pkb = kb;
-      pnb = nb;
-      pactive = A;
-      parity ^= 1;
+      // steps past every problem's rows do nothing (the last tile column only)
+      const int chunks = batch_chunks(n_max, ts, k, kb), nb = panel_outer_rest(ts, kb);
+      if (chunks >= 0) {
+        const int steps = std::max(1, chunks);
+        panel_step_batch_kernel<<<dim3(steps + (pactive ? 2 : 0), std::max(A, pactive)), kStepThreads,
+                                  panel_step_smem(nb), st>>>(b->tiles, ts, k, kb, steps, A, pk, pkb, pactive, parity,
+                                                             b->d_tile_base, b->d_nt, b->d_n, b->info, b->z,
+                                                             b->d_loc_base, b->scratch);
+        ++b->launches_per_eval;
+        pk = k;
+        pkb = kb;
+        pactive = A;
+        parity ^= 1;
+      }
       if (nb == 0) {
         const int rc = launch_jobs(b, b->panel_launch[li++]);
         if (rc != EGS_OK) return rc;
@@ -315,9 +326,9 @@ int enqueue_batch_eval(egs_batch* b) {
     const int rc = launch_jobs(b, b->trail_launch[k]);
     if (rc != EGS_OK) return rc;
   }
-  panel_step_batch_kernel<<<dim3(1 + pnb, pactive), kStepThreads, 0, st>>>(
-      b->tiles, ts, 0, 0, 0, 0, 0, pk, pkb, pnb, pactive, parity, b->d_tile_base, b->d_nt, b->info, b->z,
-      b->d_loc_base, b->scratch);
+  panel_step_batch_kernel<<<dim3(2, pactive), kStepThreads, 0, st>>>(b->tiles, ts, 0, 0, 0, 0, pk, pkb, pactive, parity,
+                                                                     b->d_tile_base, b->d_nt, b->d_n, b->info, b->z,
+                                                                     b->d_loc_base, b->scratch);
   ++b->launches_per_eval;
   logdet_batch_kernel<<<dim3(b->nt_max, b->B), 256, 0, st>>>(b->tiles, ts, b->d_tile_base, b->d_nt, b->d_n,
                                                              b->partial, b->d_partial_base);

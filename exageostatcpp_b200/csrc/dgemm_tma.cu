@@ -437,14 +437,15 @@ static int launch_desc(const void* tmap, double* tiles, GemmDesc& d, int* err, c
   return launch_cfg<false>(d.cfg, tmap, tiles, d, GemmJobs{nullptr, nullptr, 0, 0}, d.total, err, st);
 }
 
-// Trailing update of step k: C(i, j) -= L(i, k) L(j, k)^T for all k < j <= i.
-int launch_gemm_trailing(const void* tmap, double* tiles, int ts, int nt, int k, int* err, cudaStream_t st) {
+// Trailing update of step k: C(i, j) -= L(i, k) L(j, k)^T for all k < j <= i, on the
+// first `rows` rows and columns.
+int launch_gemm_trailing(const void* tmap, double* tiles, int ts, int nt, int rows, int k, int* err, cudaStream_t st) {
   GemmDesc d{};
   d.ts = ts;
   d.nt = nt;
   d.np = nt * ts;
   const int r0 = (k + 1) * ts;
-  d.M = d.N = d.np - r0;
+  d.M = d.N = rows - r0;
   d.K = ts;
   d.a_row0 = d.b_row0 = d.c_row0 = d.c_col0 = r0;
   d.a_col0 = d.b_col0 = 0;
@@ -454,8 +455,9 @@ int launch_gemm_trailing(const void* tmap, double* tiles, int ts, int nt, int k,
 }
 
 // Update of step k of the band approximation: tiles (m, c), k < c < k + band,
-// c <= m < c + band, in one launch.
-int launch_gemm_band(const void* tmap, double* tiles, int ts, int nt, int k, int band, int* err, cudaStream_t st) {
+// c <= m < c + band, in one launch, on the first `rows` rows and columns.
+int launch_gemm_band(const void* tmap, double* tiles, int ts, int nt, int rows, int k, int band, int* err,
+                     cudaStream_t st) {
   GemmDesc d{};
   d.ts = ts;
   d.nt = nt;
@@ -463,8 +465,8 @@ int launch_gemm_band(const void* tmap, double* tiles, int ts, int nt, int k, int
   const int r0 = (k + 1) * ts;
   const int cend = nt < k + band ? nt : k + band;               // columns: tiles k+1 .. cend-1
   const int rend = nt < cend - 1 + band ? nt : cend - 1 + band;  // rows: up to tile rend-1
-  d.M = rend * ts - r0;
-  d.N = cend * ts - r0;
+  d.M = (rend * ts < rows ? rend * ts : rows) - r0;
+  d.N = (cend * ts < rows ? cend * ts : rows) - r0;
   d.K = ts;
   d.a_row0 = d.b_row0 = d.c_row0 = d.c_col0 = r0;
   d.a_tcol = d.b_tcol = k;

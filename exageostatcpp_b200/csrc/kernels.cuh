@@ -37,8 +37,10 @@ struct PanelChain {
   double* z = nullptr;
 };
 long long panel_scratch_doubles();
-// 64-column blocks from column kb (a multiple of 64) of a ts-wide tile to the end of its outer block.
-int panel_outer_blocks(int ts, int kb);
+// Rows (and columns) of a problem of n points that take part in factorisations and
+// solves: the 64-row blocks with a real row.  The padding beyond them is the
+// identity and stays it.
+__host__ __device__ inline int factor_rows(int n) { return (n + 63) / 64 * 64; }
 // One step: col is tile (k, k) of a contiguous tile column, rows_below the rows
 // under the 64 x 64 block at (kb, kb), nb the further 64-column blocks of its
 // outer block (updated by the step), gcol the global column of the block (for
@@ -49,10 +51,10 @@ int launch_panel_step(double* col, int ts, int rows_below, int kb, int nb, int g
                       PanelChain& ch, cudaStream_t st);
 int launch_panel_flush(PanelChain& ch, cudaStream_t st);
 // Triangular solves against a finished factor (solve.cu): one vector in place
-// (scratch: 128 doubles), or the rows of a matrix.
-int launch_vec_forward(const double* tiles, int ts, int nt, double* z, double* scratch, cudaStream_t st,
+// of `rows` entries (a multiple of 64; scratch: 128 doubles), or the rows of a matrix.
+int launch_vec_forward(const double* tiles, int ts, int nt, int rows, double* z, double* scratch, cudaStream_t st,
                        long long* launches);
-int launch_vec_backward(const double* tiles, int ts, int nt, double* z, double* scratch, cudaStream_t st,
+int launch_vec_backward(const double* tiles, int ts, int nt, int rows, double* z, double* scratch, cudaStream_t st,
                         long long* launches);
 int launch_rows_forward(const double* tiles, int ts, int nt, double* Y, double* X, long long ldy, int rows,
                         cudaStream_t st);
@@ -111,8 +113,9 @@ int launch_gemm_batched(const void* tmap, double* tiles, int cfg, const GemmDesc
 int gemm_init_tensor_map(void* tmap_storage, double* tiles, int ts, long long ntiles);
 // The driver's cuTensorMapEncodeTiled (looked up once).
 int tensor_map_encoder(void** fn);
-int launch_gemm_trailing(const void* tmap, double* tiles, int ts, int nt, int k, int* err, cudaStream_t st);
-int launch_gemm_band(const void* tmap, double* tiles, int ts, int nt, int k, int band, int* err, cudaStream_t st);
+int launch_gemm_trailing(const void* tmap, double* tiles, int ts, int nt, int rows, int k, int* err, cudaStream_t st);
+int launch_gemm_band(const void* tmap, double* tiles, int ts, int nt, int rows, int k, int band, int* err,
+                     cudaStream_t st);
 int launch_gemm_rows(const void* tmap, double* tiles, int ts, int nt, int M, int N, int K, int a_row0,
                      int a_col0, int a_tcol, int b_row0, int b_col0, int b_tcol, int c_row0, int c_col0,
                      int lower, int* err, cudaStream_t st);

@@ -53,6 +53,13 @@ constexpr int kScratchLd = kStepMaxBlocks * kStep;
 constexpr int kScratchSlot = kScratchLd * kStep + kStep;  // solved rows, then z_k
 constexpr int kScratchDoubles = 2 * kScratchSlot;
 
+// Further 64-column blocks (0 or 1) in the outer block of column kb of a tile
+// with cols columns: outer blocks are pairs, the last one may be a single block.
+__host__ __device__ constexpr int panel_outer_rest(int cols, int kb) {
+  return ((kb / kStep) & 1) == 0 && kb + kStep < cols ? 1 : 0;
+}
+static_assert(kStepMaxBlocks == 2, "panel_outer_rest pairs the blocks");
+
 // Dynamic shared memory of a step with nb further blocks in its outer block:
 // the diagonal block, the CTA's rows, nb other row chunks, 1/L_jj and z_k.
 __host__ __device__ constexpr int panel_step_smem(int nb) {

@@ -49,20 +49,6 @@ panel_flush_kernel(const double* __restrict__ slot, double* __restrict__ col, in
 
 long long panel_scratch_doubles() { return kScratchDoubles; }
 
-int panel_outer_blocks(int ts, int kb) {
-  // a tile's 64-column blocks in as few outer blocks of at most
-  // kStepMaxBlocks as possible, of nearly equal size
-  const int nblk = ts / kStep, parts = (nblk + kStepMaxBlocks - 1) / kStepMaxBlocks;
-  const int q = nblk / parts, rem = nblk % parts, at = kb / kStep;
-  int lo = 0;
-  for (int i = 0; i < parts; ++i) {
-    const int w = q + (i < rem ? 1 : 0);
-    if (at < lo + w) return lo + w - at;
-    lo += w;
-  }
-  return 1;
-}
-
 int launch_panel_step(double* col, int ts, int rows_below, int kb, int nb, int gcol, int* info, double* z,
                       PanelChain& ch, cudaStream_t st) {
   static std::once_flag done[64];

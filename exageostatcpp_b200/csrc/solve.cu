@@ -149,8 +149,9 @@ __global__ void vec_last_kernel(const double* __restrict__ prev, double* __restr
 }
 
 template <bool kBack>
-int vec_solve(const double* tiles, int ts, int nt, double* z, double* scratch, cudaStream_t st, long long* launches) {
-  const int per = ts / kStep, steps = nt * per;
+int vec_solve(const double* tiles, int ts, int nt, int rows, double* z, double* scratch, cudaStream_t st,
+              long long* launches) {
+  const int per = ts / kStep, steps = rows / kStep;
   const double* prev = nullptr;
   double* pz = nullptr;
   for (int i = 0; i < steps; ++i) {
@@ -433,14 +434,15 @@ int rows_solve(const double* tiles, int ts, int nt, double* Y, double* X, long l
 
 }  // namespace
 
-// z := L^-1 z / L^-T z for the nt x nt lower tiles; scratch holds 128 doubles.
-int launch_vec_forward(const double* tiles, int ts, int nt, double* z, double* scratch, cudaStream_t st,
+// z := L^-1 z / L^-T z for the first `rows` rows of the nt x nt lower tiles; scratch
+// holds 128 doubles.
+int launch_vec_forward(const double* tiles, int ts, int nt, int rows, double* z, double* scratch, cudaStream_t st,
                        long long* launches) {
-  return vec_solve<false>(tiles, ts, nt, z, scratch, st, launches);
+  return vec_solve<false>(tiles, ts, nt, rows, z, scratch, st, launches);
 }
-int launch_vec_backward(const double* tiles, int ts, int nt, double* z, double* scratch, cudaStream_t st,
+int launch_vec_backward(const double* tiles, int ts, int nt, int rows, double* z, double* scratch, cudaStream_t st,
                         long long* launches) {
-  return vec_solve<true>(tiles, ts, nt, z, scratch, st, launches);
+  return vec_solve<true>(tiles, ts, nt, rows, z, scratch, st, launches);
 }
 
 // The same for `rows` (a multiple of 64) right-hand sides held as the rows of Y
