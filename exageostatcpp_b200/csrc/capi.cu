@@ -564,12 +564,12 @@ int enqueue_eval(egs_problem* p) {
   rc = p->band > 0 ? enqueue_potrf_band(p) : enqueue_potrf(p, p->z);
   if (rc != EGS_OK) return rc;
   sp = span_begin(p, EGS_STAGE_REDUCE);
-  launch_logdet_partials(p->tiles, p->ts, p->nt, p->n, p->partial, st);
+  if ((rc = launch_logdet_partials(p->tiles, p->ts, p->nt, p->n, p->partial, st)) != EGS_OK) return rc;
   span_end(p, sp, 0.0);
   count_launches(p, EGS_STAGE_REDUCE, 1);
   if (p->band > 0 && (rc = enqueue_trsv(p)) != EGS_OK) return rc;
   sp = span_begin(p, EGS_STAGE_REDUCE);
-  launch_finalize(p->partial, p->nt, p->z, p->n, p->result, p->flags, st);
+  if ((rc = launch_finalize(p->partial, p->nt, p->z, p->n, p->result, p->flags, st)) != EGS_OK) return rc;
   span_end(p, sp, 0.0);
   count_launches(p, EGS_STAGE_REDUCE, 1);
   EGS_CUDA_TRY(cudaMemcpyAsync(p->hflags, p->flags, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -645,9 +645,8 @@ static int enqueue_mixed_tail(egs_problem* p) {
 
 // Short panel of step k on stream s: gather the diagonal tile, the band tiles
 // and an identity tile into W2, factor and solve them with the FP64 panel
-// kernels (the identity row becomes L_kk^-T), scatter back.  max_ctas bounds
-// the persistent update kernels of the panel (look-ahead on spare SMs).
-static int enqueue_short_panel(egs_problem* p, int k, cudaStream_t s, int max_ctas) {
+// kernels (the identity row becomes L_kk^-T), scatter back.
+static int enqueue_short_panel(egs_problem* p, int k, cudaStream_t s) {
   const int ts = p->ts, nt = p->nt, b = p->mband;
   const int nb = std::min(b, nt - k - 1);
   int sp = span_begin(p, EGS_STAGE_PANEL, s);
@@ -678,7 +677,7 @@ int enqueue_eval_mixed_ozaki(egs_problem* p) {
   const int ts = p->ts, nt = p->nt, b = p->mband;
   int* err = p->flags + 1;
   if (int rc = enqueue_mixed_head(p)) return rc;
-  if (int rc = enqueue_short_panel(p, 0, st, 0)) return rc;
+  if (int rc = enqueue_short_panel(p, 0, st)) return rc;
   for (int k = 0; k < nt; ++k) {
     const int ntp = nt - k;
     const int nb = std::min(b, ntp - 1);
@@ -721,12 +720,12 @@ int enqueue_eval_mixed_ozaki(egs_problem* p) {
       // look-ahead: the next short panel beside the off-band update
       EGS_CUDA_TRY(cudaEventRecord(p->ev_band, st));
       EGS_CUDA_TRY(cudaStreamWaitEvent(side, p->ev_band, 0));
-      if (int rc = enqueue_short_panel(p, k + 1, side, la)) return rc;
+      if (int rc = enqueue_short_panel(p, k + 1, side)) return rc;
       EGS_CUDA_TRY(cudaEventRecord(p->ev_panel, side));
       if (int rc = enqueue_offband_update(p, k, st, gemm_num_sms() - la)) return rc;
     } else {
       if (int rc = enqueue_offband_update(p, k, st, 0)) return rc;
-      if (int rc = enqueue_short_panel(p, k + 1, st, 0)) return rc;
+      if (int rc = enqueue_short_panel(p, k + 1, st)) return rc;
       EGS_CUDA_TRY(cudaEventRecord(p->ev_panel, st));
     }
   }
@@ -1375,10 +1374,9 @@ int egs_trsv(egs_problem* p) {
 int egs_loglik_parts(egs_problem* p, double* loglik, double* logdet, double* dot) {
   if (!p) return EGS_ERR_INVALID;
   if (int rc = reject_mixed(p, "egs_loglik_parts")) return rc;
-  launch_logdet_partials(p->tiles, p->ts, p->nt, p->n, p->partial, p->stream);
-  launch_finalize(p->partial, p->nt, p->z, p->n, p->result, nullptr, p->stream);
-  int rc = check_cuda("egs_loglik_parts");
+  int rc = launch_logdet_partials(p->tiles, p->ts, p->nt, p->n, p->partial, p->stream);
   if (rc != EGS_OK) return rc;
+  if ((rc = launch_finalize(p->partial, p->nt, p->z, p->n, p->result, nullptr, p->stream)) != EGS_OK) return rc;
   EGS_CUDA_TRY(cudaMemcpyAsync(p->hresult, p->result, 4 * sizeof(double), cudaMemcpyDeviceToHost, p->stream));
   EGS_CUDA_TRY(cudaStreamSynchronize(p->stream));
   if (loglik) *loglik = p->hresult[0];
@@ -1682,8 +1680,8 @@ int egs_mle_eval_noalloc(int n, int dts, const double* x, const double* y, const
   }
   if ((rc = launch_matern_tiles(q.tiles, q.x, q.y, n, q.ts, q.nt, dparams, ktab, st)) != EGS_OK) return rc;
   if ((rc = enqueue_potrf(&q, q.z)) != EGS_OK) return rc;
-  launch_logdet_partials(q.tiles, q.ts, q.nt, n, partial, st);
-  launch_finalize(partial, q.nt, q.z, n, result, flags, st);
+  if ((rc = launch_logdet_partials(q.tiles, q.ts, q.nt, n, partial, st)) != EGS_OK) return rc;
+  if ((rc = launch_finalize(partial, q.nt, q.z, n, result, flags, st)) != EGS_OK) return rc;
   if ((rc = check_cuda("egs_mle_eval_noalloc")) != EGS_OK) return rc;
   double hres[4];
   int hflags[2];

@@ -64,9 +64,9 @@ int launch_rows_times_lower(const double* tiles, int ts, int nt, const double* W
                             cudaStream_t st);
 void launch_rows_dot(const double* A, const double* B, long long ldy, int np, int m, double* out, int stride,
                      cudaStream_t st);
-void launch_logdet_partials(const double* tiles, int ts, int nt, int n, double* partial, cudaStream_t st);
-void launch_finalize(const double* partial, int nt, const double* z, int n, double* result,
-                     const int* info, cudaStream_t st);
+int launch_logdet_partials(const double* tiles, int ts, int nt, int n, double* partial, cudaStream_t st);
+int launch_finalize(const double* partial, int nt, const double* z, int n, double* result, const int* info,
+                    cudaStream_t st);
 void launch_sumsq_diff(const double* a, const double* b, int n, double* out, cudaStream_t st);
 void launch_trmv(const double* tiles, int ts, int nt, const double* e, double* part, double* z, cudaStream_t st);
 void launch_gemv_t_block(const double* a, long long lda, int rows, int cols, const double* w, double* out,

@@ -96,9 +96,9 @@ logdet_partials_kernel(const double* __restrict__ tiles, int ts, int nt, int n, 
   if (threadIdx.x == 0) partial[k] = s;
 }
 
-void launch_logdet_partials(const double* tiles, int ts, int nt, int n, double* partial, cudaStream_t st) {
-  launch_overlapped("logdet_partials_kernel", logdet_partials_kernel, dim3(nt), dim3(256), 0, st, tiles, ts, nt, n,
-                    partial);
+int launch_logdet_partials(const double* tiles, int ts, int nt, int n, double* partial, cudaStream_t st) {
+  return launch_overlapped("logdet_partials_kernel", logdet_partials_kernel, dim3(nt), dim3(256), 0, st, tiles, ts, nt, n,
+                           partial);
 }
 
 // result = (log-likelihood, log|C|, Z^T C^-1 Z after the solve, info) (finalize_body).
@@ -109,9 +109,10 @@ finalize_kernel(const double* __restrict__ partial, int nt, const double* __rest
   finalize_body(partial, nt, z, n, result, info);
 }
 
-void launch_finalize(const double* partial, int nt, const double* z, int n, double* result, const int* info,
-                     cudaStream_t st) {
-  launch_overlapped("finalize_kernel", finalize_kernel, dim3(1), dim3(256), 0, st, partial, nt, z, n, result, info);
+int launch_finalize(const double* partial, int nt, const double* z, int n, double* result, const int* info,
+                    cudaStream_t st) {
+  return launch_overlapped("finalize_kernel", finalize_kernel, dim3(1), dim3(256), 0, st, partial, nt, z, n, result,
+                           info);
 }
 
 // out[0] = sum (a - b)^2 (DMSECodelet, dmse-codelet.cpp:60-73), fixed order.

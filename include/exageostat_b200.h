@@ -267,7 +267,7 @@ EGS_API int egs_problem_stage_stats(egs_problem* p, double* ms, double* flops, l
  * memory, work is the 16-byte aligned device workspace (overwritten), and the
  * log-likelihood is written to the host double *loglik.  It calls no
  * cudaMalloc, cudaFree or other allocating routine: its small per-call state
- * lives in one static device array of about 41 KB that every GPU which loads
+ * lives in one static device array of about 173 KB that every GPU which loads
  * the library keeps until the process exits.  The first call on a device looks
  * up that array's device address, so make this first call before any stream
  * capture.  All calls share the array: calls whose work overlaps on the GPU
