@@ -97,8 +97,8 @@ logdet_partials_kernel(const double* __restrict__ tiles, int ts, int nt, int n, 
 }
 
 int launch_logdet_partials(const double* tiles, int ts, int nt, int n, double* partial, cudaStream_t st) {
-  return launch_overlapped("logdet_partials_kernel", logdet_partials_kernel, dim3(nt), dim3(256), 0, st, tiles, ts, nt, n,
-                           partial);
+  return launch_overlapped("logdet_partials_kernel", logdet_partials_kernel, dim3(nt), dim3(256), 0, st,
+                           tiles, ts, nt, n, partial);
 }
 
 // result = (log-likelihood, log|C|, Z^T C^-1 Z after the solve, info) (finalize_body).
