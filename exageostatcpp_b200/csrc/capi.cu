@@ -687,8 +687,9 @@ int enqueue_eval_mixed_ozaki(egs_problem* p) {
     const egs_problem::OzLaunch& T = p->oz_trsm_launch[k];
     if (T.count > 0) {
       const long long srows = (long long)p->np + ts;
-      launch_ozaki_slice_f32(offband_tile(p->off_pool, ts, nt, b, k + nb + 1, k), ts, T.count, k + nb + 1,
-                             p->oz_scale, p->oz_slices, srows, st);
+      if (int rc = launch_ozaki_slice_f32(offband_tile(p->off_pool, ts, nt, b, k + nb + 1, k), ts, T.count, k + nb + 1,
+                                          p->oz_scale, p->oz_slices, srows, st))
+        return rc;
       launch_ozaki_slice_rows(p->W2 + (size_t)(nb + 1) * ts * ts, ts, p->np, p->oz_scale, p->oz_slices, srows, st);
       if (int rc = launch_ozaki_trsm(p->tm_oz, p->oz_trsm_targets + T.off, T.count, T.items, ts, k, p->np, p->W,
                                      p->oz_scale, err, st))
@@ -699,8 +700,9 @@ int enqueue_eval_mixed_ozaki(egs_problem* p) {
     if (ntp > 1) {
       // one read of the solved rows: FP16 hi/lo for the off-band update, int8
       // slices for the band update
-      launch_panel_prepare(p->W, ts, 1, ntp - 1, k, p->oz_scale, p->oz_slices, (long long)p->np + ts,
-                           p->inv_scale, p->ph, p->pl, st);
+      if (int rc = launch_panel_prepare(p->W, ts, 1, ntp - 1, k, p->oz_scale, p->oz_slices, (long long)p->np + ts,
+                                        p->inv_scale, p->ph, p->pl, st))
+        return rc;
       nl += 1;
     }
     count_launches(p, EGS_STAGE_PANEL, nl);

@@ -86,97 +86,120 @@ constexpr uint32_t idesc_i8(int n) {
 
 // Row scales and int8 slices -- and, with kSplit, the FP16 split scales and
 // hi/lo parts -- of ntiles column-major tiles (tiles0 + t ts^2, global tile row
-// row_tile0 + t), in one kernel: one CTA per 64-row strip of a tile reads the
-// strip once for its row maxima, then again in 64 x 64 blocks, transposed
-// through shared memory into the row-major (K contiguous) outputs
-// slices[p][row][c] and Ph / Pl[row][c].
+// row_tile0 + t): row-major (K contiguous) outputs slices[p][row][c] and
+// Ph / Pl[row][c].
+//
+// HBM bounds it (8 or 4 B read, 11 or 6 B written per element).  One CTA takes
+// the rows of a tile that fill 64 bytes of a column (8 FP64, 16 FP32) and keeps
+// the strip in shared memory between the row maxima and the slicing, so the tile
+// is read once; 64 KB at ts = 1,024 leave three CTAs per SM, one loading while
+// another slices, and a launch of one tile still has 128 (64) CTAs.
+// A 64-row strip read twice in 64 x 64 blocks, 16 CTAs per tile: 64 us for one
+// FP64 tile of 1,024, 186 us for 19; now 11 and 98 us (3.9 TB/s, the stores and
+// the slicing's integer work about even).  FP32: 48 and 77 (17 tiles) to 14 and 62.
+// Columns past kHeldColumns do not fit and are read again.
+//
+// Shared memory: column c at (c 64 + (c / 16) 32) bytes.  A thread slices 16
+// columns of one row; a warp covers rows of 32 bytes x chunks of 32 bytes'
+// skew, so its 32 loads touch every bank once per 128 bytes.
+constexpr int kHeldColumns = 3072;
+constexpr int prepare_smem_bytes(int ts) {
+  const int held = ts < kHeldColumns ? ts : kHeldColumns;
+  return held * 64 + held / 16 * 32;
+}
+
 template <typename T, bool kSplit, int NP>
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(256, 3)
 panel_prepare_kernel(const T* __restrict__ tiles0, int ts, int row_tile0, double* __restrict__ oz_scale,
                      int8_t* __restrict__ slices, long long slice_stride, float* __restrict__ inv_scale,
                      __half* __restrict__ Ph, __half* __restrict__ Pl) {
-  __shared__ double Sm[64][65];
-  __shared__ double red[4][64];
-  __shared__ double s_oz[64], s_f16[64];
+  constexpr int kRows = 64 / (int)sizeof(T);       // rows of the strip
+  constexpr int kWarpRows = 32 / (int)sizeof(T);   // rows x 16-column chunks of one warp's slicing step
+  constexpr int kWarpChunks = 32 / kWarpRows;
+  constexpr int kColStep = 256 / kRows;            // columns loaded by one instruction of the CTA
+  extern __shared__ __align__(16) unsigned char strip_raw[];
+  T* strip = reinterpret_cast<T*>(strip_raw);
+  __shared__ T red[8][kRows];
+  __shared__ double s_oz[kRows], s_f16[kRows];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int t = blockIdx.y;
-  const int r0 = blockIdx.x * 64;
-  const T* src = tiles0 + (long long)t * ts * ts;
+  const int r0 = blockIdx.x * kRows;
+  const T* src = tiles0 + (long long)t * ts * ts + r0;
   const long long grow0 = (long long)(row_tile0 + t) * ts + r0;
+  const int held = ts < kHeldColumns ? ts : kHeldColumns;
   {
-    const int rl = threadIdx.x & 63, g = threadIdx.x >> 6;
-    const T* col = src + r0 + rl;
-    double m0 = 0.0, m1 = 0.0, m2 = 0.0, m3 = 0.0;  // ts is a multiple of 64
-#pragma unroll 4
-    for (int c = g; c < ts; c += 16) {
-      m0 = fmax(m0, fabs((double)col[(long long)c * ts]));
-      m1 = fmax(m1, fabs((double)col[(long long)(c + 4) * ts]));
-      m2 = fmax(m2, fabs((double)col[(long long)(c + 8) * ts]));
-      m3 = fmax(m3, fabs((double)col[(long long)(c + 12) * ts]));
+    const int r = tid % kRows;
+    T m = T(0);
+#pragma unroll 16
+    for (int c = tid / kRows; c < held; c += kColStep) {
+      const T v = src[(long long)c * ts + r];
+      strip[c * kRows + (c >> 4) * kWarpRows + r] = v;
+      m = fmax(m, fabs(v));
     }
-    red[g][rl] = fmax(fmax(m0, m1), fmax(m2, m3));
-    __syncthreads();
-    if (g == 0) {
-      const double m = fmax(fmax(red[0][rl], red[1][rl]), fmax(red[2][rl], red[3][rl]));
-      const double so = oz_row_scale(m);
-      oz_scale[grow0 + rl] = so;
-      s_oz[rl] = (so > 0.0) ? 1.0 / so : 0.0;  // exact: a power of two
-      if constexpr (kSplit) {
-        const float inv = f16_row_inv_scale(m);
-        inv_scale[grow0 + rl] = inv;
-        s_f16[rl] = (inv > 0.0f) ? 1.0 / (double)inv : 0.0;  // exact: a power of two
-      }
+    for (int c = held + tid / kRows; c < ts; c += kColStep) m = fmax(m, fabs(src[(long long)c * ts + r]));
+#pragma unroll
+    for (int o = 16; o >= kRows; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (lane < kRows) red[warp][lane] = m;
+  }
+  __syncthreads();
+  if (tid < kRows) {
+    T m = red[0][tid];
+#pragma unroll
+    for (int w = 1; w < 8; ++w) m = fmax(m, red[w][tid]);
+    const double so = oz_row_scale((double)m);
+    oz_scale[grow0 + tid] = so;
+    s_oz[tid] = (so > 0.0) ? 1.0 / so : 0.0;  // exact: a power of two
+    if constexpr (kSplit) {
+      const float inv = f16_row_inv_scale((double)m);
+      inv_scale[grow0 + tid] = inv;
+      s_f16[tid] = (inv > 0.0f) ? 1.0 / (double)inv : 0.0;  // exact: a power of two
     }
   }
-  // Pass 2, 64 x 64 blocks; the next block's loads are issued before the
-  // current block is split.  Without kSplit every thread slices 16 columns of
-  // one row; with kSplit warps 0-3 slice and warps 4-7 split to FP16, 2 x 16
-  // columns of one row per thread, so neither needs both sets of registers.
-  T w[16];
+  __syncthreads();
+  const int chunks = ts / 16;
+  constexpr int kGroups = kRows / kWarpRows;
+  for (int task = warp;; task += 8) {
+    const int r = (task % kGroups) * kWarpRows + lane % kWarpRows;
+    const int first = (task / kGroups) * kWarpChunks;
+    if (first >= chunks) break;
+    const int chunk = first + lane / kWarpRows;  // < chunks: ts is a multiple of 128
+    const int c0 = chunk * 16;
+    const long long off = (grow0 + r) * ts + c0;
+    T x[16];
+    if (c0 < held) {
+      const T* s = strip + c0 * kRows + chunk * kWarpRows + r;
 #pragma unroll
-  for (int q = 0; q < 16; ++q) {
-    const int e = q * 256 + threadIdx.x;
-    w[q] = src[(long long)(e >> 6) * ts + r0 + (e & 63)];
-  }
-  for (int c0 = 0; c0 < ts; c0 += 64) {
-    __syncthreads();  // Sm free; the scales are visible
-#pragma unroll
-    for (int q = 0; q < 16; ++q) {
-      const int e = q * 256 + threadIdx.x;
-      Sm[e & 63][e >> 6] = (double)w[q];
-    }
-    if (c0 + 64 < ts) {
-#pragma unroll
-      for (int q = 0; q < 16; ++q) {
-        const int e = q * 256 + threadIdx.x;
-        w[q] = src[(long long)(c0 + 64 + (e >> 6)) * ts + r0 + (e & 63)];
-      }
-    }
-    __syncthreads();
-    if constexpr (!kSplit) {
-      const int r = threadIdx.x >> 2, cq = (threadIdx.x & 3) * 16;
-      const double io = s_oz[r];
-      double v[16];
-#pragma unroll
-      for (int c = 0; c < 16; ++c) v[c] = Sm[r][cq + c] * io;  // |v| < 1
-      oz_emit_slices<NP>(v, slices + (grow0 + r) * ts + c0 + cq, slice_stride);
+      for (int c = 0; c < 16; ++c) x[c] = s[c * kRows];
     } else {
-      const int tt = threadIdx.x & 127, r = tt >> 1;
-      const bool to_f16 = threadIdx.x >= 128;  // warp-uniform
-      const double sc = to_f16 ? s_f16[r] : s_oz[r];
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int cq = (tt & 1) * 32 + h * 16;
-        const long long off = (grow0 + r) * ts + c0 + cq;
-        double v[16];
-#pragma unroll
-        for (int c = 0; c < 16; ++c) v[c] = Sm[r][cq + c] * sc;
-        if (to_f16)
-          f16_emit_split(v, Ph + off, Pl + off);
-        else
-          oz_emit_slices<NP>(v, slices + off, slice_stride);  // |v| < 1
-      }
+      for (int c = 0; c < 16; ++c) x[c] = src[(long long)(c0 + c) * ts + r];
     }
+    double v[16];
+    if constexpr (kSplit) {
+      const double sf = s_f16[r];
+#pragma unroll
+      for (int c = 0; c < 16; ++c) v[c] = (double)x[c] * sf;
+      f16_emit_split(v, Ph + off, Pl + off);
+    }
+    const double so = s_oz[r];
+#pragma unroll
+    for (int c = 0; c < 16; ++c) v[c] = (double)x[c] * so;  // |v| < 1
+    oz_emit_slices<NP>(v, slices + off, slice_stride);
   }
+}
+
+template <typename T, bool kSplit, int NP>
+static int launch_prepare(const T* tiles0, int ts, int ntiles, int row_tile0, double* oz_scale, int8_t* slices,
+                          long long rows, float* inv_scale, __half* Ph, __half* Pl, cudaStream_t st) {
+  if (ntiles <= 0) return EGS_OK;
+  static std::once_flag attr_done[64];
+  once_per_device(attr_done, []() {
+    cudaFuncSetAttribute(panel_prepare_kernel<T, kSplit, NP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         prepare_smem_bytes(kHeldColumns));
+  });
+  panel_prepare_kernel<T, kSplit, NP><<<dim3(ts * (int)sizeof(T) / 64, ntiles), 256, prepare_smem_bytes(ts), st>>>(
+      tiles0, ts, row_tile0, oz_scale, slices, rows * (long long)ts, inv_scale, Ph, Pl);
+  return launch_status("panel_prepare_kernel");
 }
 
 // Row scale of ts rows stored row by row (row r at src + r ts), written to
@@ -587,28 +610,25 @@ int ozaki_tensor_map(void* storage, const int8_t* slices, int ts, long long rows
 }
 
 // Panel tiles W[t0 .. t0+ntiles) = global tile rows row_tile0 + t0 .. (column-major FP64).
-void launch_ozaki_slice(const double* W, int ts, int t0, int ntiles, int row_tile0, double* scale, int8_t* slices,
+int launch_ozaki_slice(const double* W, int ts, int t0, int ntiles, int row_tile0, double* scale, int8_t* slices,
                         long long rows, cudaStream_t st) {
-  if (ntiles <= 0) return;
-  panel_prepare_kernel<double, false, kOzSlices><<<dim3(ts / 64, ntiles), 256, 0, st>>>(
-      W + (long long)t0 * ts * ts, ts, row_tile0 + t0, scale, slices, rows * (long long)ts, nullptr, nullptr, nullptr);
+  return launch_prepare<double, false, kOzSlices>(W + (long long)t0 * ts * ts, ts, ntiles, row_tile0 + t0, scale,
+                                                  slices, rows, nullptr, nullptr, nullptr, st);
 }
 
 // As launch_ozaki_slice, plus the FP16 split (inv_scale, Ph, Pl) of the same
 // rows for the split-FP16 update, from one read of the panel.
-void launch_panel_prepare(const double* W, int ts, int t0, int ntiles, int row_tile0, double* oz_scale,
+int launch_panel_prepare(const double* W, int ts, int t0, int ntiles, int row_tile0, double* oz_scale,
                           int8_t* slices, long long rows, float* inv_scale, __half* Ph, __half* Pl, cudaStream_t st) {
-  if (ntiles <= 0) return;
-  panel_prepare_kernel<double, true, kOzSlices><<<dim3(ts / 64, ntiles), 256, 0, st>>>(
-      W + (long long)t0 * ts * ts, ts, row_tile0 + t0, oz_scale, slices, rows * (long long)ts, inv_scale, Ph, Pl);
+  return launch_prepare<double, true, kOzSlices>(W + (long long)t0 * ts * ts, ts, ntiles, row_tile0 + t0, oz_scale,
+                                                 slices, rows, inv_scale, Ph, Pl, st);
 }
 
 // Contiguous FP32 column-major tiles (global tile rows row_tile0 ..).
-void launch_ozaki_slice_f32(const float* tiles0, int ts, int ntiles, int row_tile0, double* scale, int8_t* slices,
+int launch_ozaki_slice_f32(const float* tiles0, int ts, int ntiles, int row_tile0, double* scale, int8_t* slices,
                             long long rows, cudaStream_t st) {
-  if (ntiles <= 0) return;
-  panel_prepare_kernel<float, false, kOzPanelSlices><<<dim3(ts / 64, ntiles), 256, 0, st>>>(
-      tiles0, ts, row_tile0, scale, slices, rows * (long long)ts, nullptr, nullptr, nullptr);
+  return launch_prepare<float, false, kOzPanelSlices>(tiles0, ts, ntiles, row_tile0, scale, slices, rows, nullptr,
+                                                      nullptr, nullptr, st);
 }
 
 // ts rows stored row by row at src into slice rows row0 .. row0 + ts.
@@ -732,7 +752,7 @@ extern "C" int egs_ozaki_band_update(int ts, int nt, int band, int k, const doub
   cudaMemset(sl, 0, (size_t)rows * ts * oz::S);
   if (!targets.empty()) cudaMemcpy(dt, targets.data(), targets.size() * sizeof(int4), cudaMemcpyHostToDevice);
   if ((rc = ozaki_tensor_map(tm, sl, ts, rows)) != EGS_OK) goto done;
-  launch_ozaki_slice(W, ts, 1, ntp - 1, k, scale, sl, rows, 0);
+  if ((rc = launch_ozaki_slice(W, ts, 1, ntp - 1, k, scale, sl, rows, 0)) != EGS_OK) goto done;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
   cudaEventRecord(e0, 0);
