@@ -1954,7 +1954,7 @@ int egs_mloe_mmom_host(int n_obs, int n_miss, int dts, const double* x_obs, cons
   }
   if ((rc = sync_flags(pt, false)) != EGS_OK || (rc = sync_flags(pa, false)) != EGS_OK) return rc;
   cudaStream_t st = pa->stream, st2 = pt->stream;
-  const int ts = pa->ts, nt = pa->nt, np = pa->np;
+  const int ts = pa->ts, nt = pa->nt, np = factor_rows(n_obs), nb = np / kInnerBlock;
   // targets in groups of at most 512, as the rows of a matrix (64-row chunks)
   const int group = std::min((n_miss + kInnerBlock - 1) / kInnerBlock * kInnerBlock, 512);
   double *ya = nullptr, *xa = nullptr, *yt = nullptr, *xt = nullptr, *dxm = nullptr, *dym = nullptr, *dots = nullptr;
@@ -2000,17 +2000,17 @@ int egs_mloe_mmom_host(int n_obs, int n_miss, int dts, const double* x_obs, cons
     cudaEventRecord(ready, st);
     cudaStreamWaitEvent(st2, ready, 0);
     // L_t^-1 k_t beside L_a^-1 [k_a, k_t] = [y_a, y_t]
-    if ((rc = launch_rows_forward(pt->tiles, ts, nt, yt, xt, ldt, group, st2)) != EGS_OK ||
-        (rc = launch_rows_forward(pa->tiles, ts, nt, ya, xa, lda, 2 * group, st)) != EGS_OK)
+    if ((rc = launch_rows_forward(pt->tiles, ts, nt, nb, yt, xt, ldt, group, st2)) != EGS_OK ||
+        (rc = launch_rows_forward(pa->tiles, ts, nt, nb, ya, xa, lda, 2 * group, st)) != EGS_OK)
       break;
     cudaEventRecord(ready, st2);
     launch_rows_dot(xa, xa, lda, np, m, d + 0, 4, st);          // k_a' K_a^-1 k_a
     launch_rows_dot(xa + group, xa, lda, np, m, d + 1, 4, st);  // k_t' K_a^-1 k_a
     // w_a = L_a^-T y_a; w_a' K_t w_a = |L_t^T w_a|^2
-    if ((rc = launch_rows_backward(pa->tiles, ts, nt, xa, ya, lda, group, st)) != EGS_OK) break;
+    if ((rc = launch_rows_backward(pa->tiles, ts, nt, nb, xa, ya, lda, group, st)) != EGS_OK) break;
     cudaStreamWaitEvent(st, ready, 0);
     launch_rows_dot(xt, xt, ldt, np, m, d + 2, 4, st);          // k_t' K_t^-1 k_t
-    if ((rc = launch_rows_times_lower(pt->tiles, ts, nt, ya, ya + group, lda, group, st)) != EGS_OK) break;
+    if ((rc = launch_rows_times_lower(pt->tiles, ts, nt, nb, ya, ya + group, lda, group, st)) != EGS_OK) break;
     launch_rows_dot(ya + group, ya + group, lda, np, m, d + 3, 4, st);
     rc = check_cuda("egs_mloe_mmom_host");
   }

@@ -8,7 +8,8 @@
 //     A_jk = 1/2 sum(M_j o M_k),   M_j = L^-1 C_j L^-T  (symmetric),
 // which needs no N^3 product per pair.  C is factored once; the rows of the three
 // symmetric C_j, stacked, go through two row solves: X_j = C_j L^-T, then X_j^T L^-T =
-// L^-1 C_j L^-T = M_j (solve.cu).
+// L^-1 C_j L^-T = M_j, of which only the lower half is computed, a third of a full
+// solve's work (solve.cu; N = 1,600: second sweep 1.02 -> 0.53 ms, the call 2.96 -> 2.54).
 //
 // Derivative kernels (src/kernels/concrete/UnivariateMaternDdsigmaSquare.cpp,
 // UnivariateMaternDbeta.cpp, UnivariateMaternDnu.cpp): at scaled distance
@@ -107,8 +108,9 @@ transpose_stacked_kernel(const double* __restrict__ X, int np, double* __restric
   for (int c = threadIdx.x >> 6; c < 64; c += 4) dst[(r0 + c) * ld + c0 + r] = t[r][c];
 }
 
-// The six sums of M_j o M_k (j <= k) over the stacked matrices: per-block partial
-// sums in a fixed order, then one warp per pair adds the partials in a fixed order.
+// The six sums of M_j o M_k (j <= k) over the lower halves of the stacked symmetric
+// matrices: per-block partial sums in a fixed order, then one warp per pair adds the
+// partials in a fixed order.
 constexpr int kPairs = 6;
 __global__ void __launch_bounds__(256)
 pair_dots_kernel(const double* __restrict__ M, int np, double* __restrict__ partial) {
@@ -116,15 +118,18 @@ pair_dots_kernel(const double* __restrict__ M, int np, double* __restrict__ part
   double acc[kPairs] = {};
   const long long nn = (long long)np * np;
   for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < nn; i += (long long)gridDim.x * 256) {
-    const long long c = i / np;
-    const double* m = M + c * 3 * np + (i - c * np);
+    const long long c = i / np, r = i - c * np;
+    if (r < c) continue;
+    const double w = (r == c) ? 1.0 : 2.0;
+    const double* m = M + c * 3 * np + r;
     const double a = m[0], b = m[np], d = m[2 * (long long)np];
-    acc[0] = fma(a, a, acc[0]);
-    acc[1] = fma(a, b, acc[1]);
-    acc[2] = fma(a, d, acc[2]);
-    acc[3] = fma(b, b, acc[3]);
-    acc[4] = fma(b, d, acc[4]);
-    acc[5] = fma(d, d, acc[5]);
+    const double wa = w * a, wb = w * b;
+    acc[0] = fma(wa, a, acc[0]);
+    acc[1] = fma(wa, b, acc[1]);
+    acc[2] = fma(wa, d, acc[2]);
+    acc[3] = fma(wb, b, acc[3]);
+    acc[4] = fma(wb, d, acc[4]);
+    acc[5] = fma(w * d, d, acc[5]);
   }
 #pragma unroll
   for (int q = 0; q < kPairs; ++q) {
@@ -197,7 +202,7 @@ extern "C" int egs_fisher_host(int n, int dts, const double* x, const double* y,
     return EGS_ERR_INVALID;
   }
   if ((rc = egs_problem_set_locations(p, x, y)) != EGS_OK || (rc = factor_resident(p, theta)) != EGS_OK) return rc;
-  const int np = nt * ts;
+  const int np = factor_rows(n);
   const size_t nn3 = 3 * (size_t)np * np;
   double *Y = nullptr, *X = nullptr, *tabs = nullptr, *part = nullptr, *dots = nullptr;
   MaternParams* orders = nullptr;
@@ -247,13 +252,13 @@ extern "C" int egs_fisher_host(int n, int dts, const double* x, const double* y,
   cudaMemcpyAsync(orders, hp, sizeof(hp), cudaMemcpyHostToDevice, st);
   launch_matern_ktab(orders, tabs, kFisherOrders, st);
   matern_derivatives_kernel<<<3 * gemm_num_sms(), 256, kFisherTabBytes, st>>>(dx, dy, n, np, q, orders, tabs, Y);
-  // Y = C_j -> X = C_j L^-T; Y = X^T = L^-1 C_j -> X = L^-1 C_j L^-T = M_j
-  if ((rc = launch_rows_forward(tiles, ts, nt, Y, X, 3LL * np, 3 * np, st)) != EGS_OK) {
+  // Y = C_j -> X = C_j L^-T; Y = X^T = L^-1 C_j -> X = L^-1 C_j L^-T = M_j, its lower half
+  if ((rc = launch_rows_forward(tiles, ts, nt, np / 64, Y, X, 3LL * np, 3 * np, st)) != EGS_OK) {
     cleanup();
     return rc;
   }
   transpose_stacked_kernel<<<dim3(np / 64, np / 64, 3), 256, 0, st>>>(X, np, Y);
-  if ((rc = launch_rows_forward(tiles, ts, nt, Y, X, 3LL * np, 3 * np, st)) != EGS_OK) {
+  if ((rc = launch_rows_forward_symmetric(tiles, ts, nt, np / 64, Y, X, 3, st)) != EGS_OK) {
     cleanup();
     return rc;
   }

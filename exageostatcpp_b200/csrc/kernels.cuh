@@ -56,12 +56,14 @@ int launch_vec_forward(const double* tiles, int ts, int nt, int rows, double* z,
                        long long* launches);
 int launch_vec_backward(const double* tiles, int ts, int nt, int rows, double* z, double* scratch, cudaStream_t st,
                         long long* launches);
-int launch_rows_forward(const double* tiles, int ts, int nt, double* Y, double* X, long long ldy, int rows,
+int launch_rows_forward(const double* tiles, int ts, int nt, int blocks, double* Y, double* X, long long ldy, int rows,
                         cudaStream_t st);
-int launch_rows_backward(const double* tiles, int ts, int nt, double* Y, double* X, long long ldy, int rows,
-                         cudaStream_t st);
-int launch_rows_times_lower(const double* tiles, int ts, int nt, const double* W, double* U, long long ldy, int rows,
-                            cudaStream_t st);
+int launch_rows_backward(const double* tiles, int ts, int nt, int blocks, double* Y, double* X, long long ldy,
+                         int rows, cudaStream_t st);
+int launch_rows_forward_symmetric(const double* tiles, int ts, int nt, int blocks, double* Y, double* X, int count,
+                                  cudaStream_t st);
+int launch_rows_times_lower(const double* tiles, int ts, int nt, int blocks, const double* W, double* U, long long ldy,
+                            int rows, cudaStream_t st);
 void launch_rows_dot(const double* A, const double* B, long long ldy, int np, int m, double* out, int stride,
                      cudaStream_t st);
 int launch_logdet_partials(const double* tiles, int ts, int nt, int n, double* partial, cudaStream_t st);

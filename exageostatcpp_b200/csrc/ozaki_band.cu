@@ -100,8 +100,8 @@ constexpr uint32_t idesc_i8(int n) {
 // Columns past kHeldColumns do not fit and are read again.
 //
 // Shared memory: column c at (c 64 + (c / 16) 32) bytes.  A thread slices 16
-// columns of one row; a warp covers rows of 32 bytes x chunks of 32 bytes'
-// skew, so its 32 loads touch every bank once per 128 bytes.
+// columns of one row; the 32 bytes of rows in a warp and the 32-byte skew of its
+// chunks make each of its loads touch every bank equally often.
 constexpr int kHeldColumns = 3072;
 constexpr int prepare_smem_bytes(int ts) {
   const int held = ts < kHeldColumns ? ts : kHeldColumns;

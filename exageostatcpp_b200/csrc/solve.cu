@@ -226,19 +226,29 @@ __device__ __forceinline__ void rows_back16(double* X, const double* D, const do
 }
 
 // Step of the 64 columns at global column r0 = k ts + kb: X_b := Y_b L_bb^-T (kBack:
-// L_bb^-1) for the 64 rows 64 blockIdx.y .., and Y_j -= X_b L_jb^T (kBack: X_b L_bj) for
-// the column blocks j = blockIdx.x, blockIdx.x + gridDim.x, .. of the nblk remaining
-// ones.  Y and X are column-major with column stride ldy.
+// L_bb^-1) for one chunk of 64 rows, and Y_j -= X_b L_jb^T (kBack: X_b L_bj) for the
+// remaining column blocks j, share of them per CTA of the row.  Y and X are
+// column-major with column stride ldy.  With sym > 0 the rows are stacked symmetric
+// results of sym chunks each, of which only the blocks on and below the diagonal are
+// wanted: the chunks above block column b are left out, the others stop at theirs.
 template <bool kBack>
 __global__ void __launch_bounds__(kRowsThreads)
-rows_step_kernel(const double* __restrict__ tiles, int ts, int nt, int k, int kb, int nblk, double* Y,
-                 double* __restrict__ X, long long ldy) {
+rows_step_kernel(const double* __restrict__ tiles, int ts, int nt, int k, int kb, int nblk, int share, int sym,
+                 double* Y, double* __restrict__ X, long long ldy) {
   extern __shared__ __align__(16) double sm[];
   double *D = sm, *A = sm + kStepBlock, *B = sm + 2 * kStepBlock, *pinv = sm + 3 * kStepBlock;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const long long ts2 = (long long)ts * ts;
   const int r0 = k * ts + kb;
-  double* Yc = Y + kStep * blockIdx.y;
+  int chunk = blockIdx.y;
+  if (sym > 0) {
+    const int left = nblk + 1;  // chunks per matrix from block column b on, the longest first
+    chunk = (blockIdx.y / left) * sym + sym - 1 - blockIdx.y % left;
+    nblk -= blockIdx.y % left;
+  }
+  const int step = (nblk + share - 1) / share;  // CTAs with blocks of this row
+  if (blockIdx.x > 0 && (int)blockIdx.x >= step) return;
+  double* Yc = Y + kStep * chunk;
   auto first_col = [&](int j) { return kBack ? kStep * j : r0 + kStep * (j + 1); };
   auto fetch_b = [&](int j) {
     const int at = first_col(j), t = at / ts, lo = at - t * ts;
@@ -266,7 +276,7 @@ rows_step_kernel(const double* __restrict__ tiles, int ts, int nt, int k, int kb
   cp_async_wait<0>();
   __syncthreads();
   if (blockIdx.x == 0) {
-    double* Xc = X + kStep * blockIdx.y;
+    double* Xc = X + kStep * chunk;
     for (int e = tid; e < kStep * kStep / 2; e += kRowsThreads) {
       const int c = e >> 5, r = 2 * (e & 31);
       *reinterpret_cast<double2*>(Xc + (r0 + c) * ldy + r) = *reinterpret_cast<const double2*>(A + c * kStepLd + r);
@@ -274,7 +284,7 @@ rows_step_kernel(const double* __restrict__ tiles, int ts, int nt, int k, int kb
   }
   const int g = lane >> 2, t = lane & 3;
 #pragma unroll 1
-  for (int j = blockIdx.x; j < nblk; j += gridDim.x) {
+  for (int j = blockIdx.x; j < nblk; j += step) {
     if (j != (int)blockIdx.x) {
       __syncthreads();  // every warp is done with the previous block of L
       fetch_b(j);
@@ -412,8 +422,10 @@ int rows_share(int nblk, int chunks) {
   return best;
 }
 
+// blocks: the 64-column blocks that take part.
 template <bool kBack>
-int rows_solve(const double* tiles, int ts, int nt, double* Y, double* X, long long ldy, int rows, cudaStream_t st) {
+int rows_solve(const double* tiles, int ts, int nt, int blocks, double* Y, double* X, long long ldy, int rows, int sym,
+               cudaStream_t st) {
   static std::once_flag done[64];
   once_per_device(done, []() {
     constexpr auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
@@ -421,13 +433,14 @@ int rows_solve(const double* tiles, int ts, int nt, double* Y, double* X, long l
     cudaFuncSetAttribute(rows_step_kernel<true>, attr, rows_step_smem());
     cudaFuncSetAttribute(rows_times_lower_kernel, attr, rows_times_smem());
   });
-  const int per = ts / kStep, steps = nt * per;
-  for (int i = 0; i < steps; ++i) {
-    const int b = kBack ? steps - 1 - i : i;
-    const int nblk = kBack ? b : steps - 1 - b;
-    const int share = rows_share(nblk, rows / kStep);
-    rows_step_kernel<kBack><<<dim3(nblk > 0 ? (nblk + share - 1) / share : 1, rows / kStep), kRowsThreads,
-                              rows_step_smem(), st>>>(tiles, ts, nt, b / per, (b % per) * kStep, nblk, Y, X, ldy);
+  const int per = ts / kStep;
+  for (int i = 0; i < blocks; ++i) {
+    const int b = kBack ? blocks - 1 - i : i;
+    const int nblk = kBack ? b : blocks - 1 - b;
+    const int chunks = sym > 0 ? rows / kStep / sym * (nblk + 1) : rows / kStep;
+    const int share = rows_share(sym > 0 ? (nblk + 1) / 2 : nblk, chunks);
+    rows_step_kernel<kBack><<<dim3(nblk > 0 ? (nblk + share - 1) / share : 1, chunks), kRowsThreads, rows_step_smem(),
+                              st>>>(tiles, ts, nt, b / per, (b % per) * kStep, nblk, share, sym, Y, X, ldy);
   }
   return launch_status("rows_step_kernel");
 }
@@ -446,21 +459,30 @@ int launch_vec_backward(const double* tiles, int ts, int nt, int rows, double* z
 }
 
 // The same for `rows` (a multiple of 64) right-hand sides held as the rows of Y
-// (column c of length ldy at Y + c ldy, np columns): X := Y L^-T / Y L^-1.  Y is overwritten.
-int launch_rows_forward(const double* tiles, int ts, int nt, double* Y, double* X, long long ldy, int rows,
+// (column c of length ldy at Y + c ldy, 64 blocks columns): X := Y L^-T / Y L^-1 by the
+// first `blocks` 64-column blocks of L.  Y is overwritten.
+int launch_rows_forward(const double* tiles, int ts, int nt, int blocks, double* Y, double* X, long long ldy, int rows,
                         cudaStream_t st) {
-  return rows_solve<false>(tiles, ts, nt, Y, X, ldy, rows, st);
+  return rows_solve<false>(tiles, ts, nt, blocks, Y, X, ldy, rows, 0, st);
 }
-int launch_rows_backward(const double* tiles, int ts, int nt, double* Y, double* X, long long ldy, int rows,
-                         cudaStream_t st) {
-  return rows_solve<true>(tiles, ts, nt, Y, X, ldy, rows, st);
+int launch_rows_backward(const double* tiles, int ts, int nt, int blocks, double* Y, double* X, long long ldy,
+                         int rows, cudaStream_t st) {
+  return rows_solve<true>(tiles, ts, nt, blocks, Y, X, ldy, rows, 0, st);
+}
+
+// X := Y L^-T for `count` stacked square matrices whose results are symmetric: only the
+// 64 x 64 blocks on and below each diagonal are computed, a third of the work.
+int launch_rows_forward_symmetric(const double* tiles, int ts, int nt, int blocks, double* Y, double* X, int count,
+                                  cudaStream_t st) {
+  const int rows = count * blocks * kStep;
+  return rows_solve<false>(tiles, ts, nt, blocks, Y, X, rows, rows, blocks, st);
 }
 
 // U := -W L for the lower tiles (after a launch_rows_* call of this process on the device).
-int launch_rows_times_lower(const double* tiles, int ts, int nt, const double* W, double* U, long long ldy, int rows,
-                            cudaStream_t st) {
-  rows_times_lower_kernel<<<dim3(nt * (ts / kStep), rows / kStep), kRowsThreads, rows_times_smem(), st>>>(tiles, ts, nt,
-                                                                                                        W, U, ldy);
+int launch_rows_times_lower(const double* tiles, int ts, int nt, int blocks, const double* W, double* U, long long ldy,
+                            int rows, cudaStream_t st) {
+  rows_times_lower_kernel<<<dim3(blocks, rows / kStep), kRowsThreads, rows_times_smem(), st>>>(tiles, ts, nt, W, U,
+                                                                                            ldy);
   return launch_status("rows_times_lower_kernel");
 }
 

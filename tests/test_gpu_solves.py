@@ -69,3 +69,16 @@ def test_fisher_orders_and_sizes(n, dts, theta):
     inv = egs.fisher_host(x, y, theta, dts)
     ref = O.fisher_inverse(x, y, theta)
     assert np.abs(inv - ref).max() <= 1e-7 * np.abs(ref).max(), (inv, ref)
+
+
+@pytest.mark.parametrize("n,dts", [(129, 64), (200, 320), (1000, 960)])
+def test_row_sweeps_end_at_the_last_real_block(n, dts):
+    # tiles mostly of padding, which the sweeps leave out, and odd numbers of the
+    # blocks that the symmetric sweep stops at; tolerances as above
+    theta = (1.1, 0.04, 0.8)
+    x, y = egs.generate_locations(n + 70, 11)
+    inv, ref = egs.fisher_host(x[:n], y[:n], theta, dts), O.fisher_inverse(x[:n], y[:n], theta)
+    assert np.abs(inv - ref).max() <= 1e-7 * np.abs(ref).max(), (inv, ref)
+    args = (x[:n], y[:n], x[n:], y[n:], theta, (0.9, 0.05, 0.7))
+    got, ref = egs.mloe_mmom_host(*args, dts), O.mloe_mmom(*args)
+    assert abs(got[0] - ref[0]) < 1e-10 and abs(got[1] - ref[1]) < 1e-10, (got, ref)
