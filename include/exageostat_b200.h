@@ -293,7 +293,7 @@ EGS_API int egs_problem_set_graphs(egs_problem* p, int enable);
  * independent problems (problem i: n[i] points, caller arrays concatenated in
  * order in x, y, z, host memory) factored with one common tile size
  * (round-up(dts, 64)).  Every stage runs once per batch: one tile pool and one
- * TMA descriptor for all problems, the 64x64 potrf, row solves and
+ * TMA descriptor for all problems, the 64-column panel steps and
  * tensor-core updates of all problems still active at step k in one launch
  * each.  From the second egs_batch_eval on, the whole batched evaluation is one
  * CUDA graph replay.  Results are the same formulas as egs_mle_eval per
