@@ -319,9 +319,21 @@ __global__ void copy_segment_kernel(const double* __restrict__ src, double* __re
   if (i < n) dst[i] = src[i];
 }
 
+// Largest tile of the solves.  Beside their static reduction buffers (12.4 and 4.3 KB)
+// their copy of a tile's vector segment passes the 48 KB that a launch has by default from
+// tiles of 4,608 on, so both kernels ask for room for it.
+constexpr int kSolveMaxTile = 5888;
+
 // v := (L L^T)^-1 v with the mixed factor; tmp holds ts doubles.
 void launch_mixed_solve(const double* band, const float* off, const double* inv, int ts, int nt, int b, double* v,
                         double* tmp, cudaStream_t st, long long* launches) {
+  static std::once_flag attr_done[64];
+  once_per_device(attr_done, []() {
+    constexpr auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    constexpr int bytes = kSolveMaxTile * (int)sizeof(double);
+    cudaFuncSetAttribute(gemv_mixed_kernel, attr, bytes);
+    cudaFuncSetAttribute(inv_apply_kernel, attr, bytes);
+  });
   const long long ts2 = (long long)ts * ts;
   for (int k = 0; k < nt; ++k) {
     inv_apply_t_kernel<<<(ts + 7) / 8, 256, 0, st>>>(inv + k * ts2, ts, v + (long long)k * ts, tmp);
