@@ -43,7 +43,8 @@
 namespace egs {
 
 constexpr int kStep = 64;           // columns of a step, rows of a chunk
-constexpr int kStepLd = 68;         // shared-memory column stride: fragment loads hit distinct banks
+constexpr int kStepLd = 68;         // shared-memory column stride: fragment loads hit distinct banks;
+                                    // the padding of the diagonal block's columns holds the pivots
 constexpr int kStepBlock = kStep * kStepLd;
 constexpr int kStepMaxBlocks = 2;   // most 64-column blocks of an outer block
 constexpr int kStepThreads = 128 * ((2 * kStepMaxBlocks + 4) / 3);
@@ -137,7 +138,9 @@ __device__ __forceinline__ void block_update_16(double* x, int row0, int n0, con
 
 // 1 / sqrt(d) for normal d well inside the exponent range: the hardware's
 // approximation y (about 2^-20) and one step of Householder's third-order
-// iteration on its residual e, y (1 + e / 2 + 3 e^2 / 8): 2^-60 before rounding.
+// iteration on its residual e, y (1 + e / 2 + 3 e^2 / 8).  The omitted 5 e^3 / 16 is
+// below 2^-58, the rounding of d y in e puts 2^-54 into the result, its own rounding
+// 2^-53: within 2^-52 of the root's reciprocal, as a rounded root and a rounded division are.
 // A shorter dependent chain than rsqrt(), which the pivots below wait for.
 __device__ __forceinline__ double step_rsqrt(double d) {
   double y;
@@ -151,12 +154,14 @@ __device__ __forceinline__ double step_rsqrt(double d) {
 // fused multiply-add.  l[j][j] becomes 1 / L_jj.  Returns a mask of the pivots outside
 // the range of the fast rsqrt (zero, negative, NaN, subnormal, huge); kSafe uses
 // rsqrt() and returns the mask of pivots that are not positive (or NaN).
+// The pivots themselves go to piv (stride kStepLd), for step_roots.
 template <bool kSafe>
-__device__ __forceinline__ unsigned step_factor8(double (&l)[8][8]) {
+__device__ __forceinline__ unsigned step_factor8(double (&l)[8][8], double* piv, int lane) {
   unsigned mask = 0;
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     const double d = l[j][j];
+    if (lane == 0) piv[j * kStepLd] = d;
     if constexpr (kSafe) {
       if (!(d > 0.0)) mask |= 1u << j;
       l[j][j] = rsqrt(d);
@@ -239,9 +244,9 @@ __device__ __forceinline__ void step_pivots8(double* D, double* pinv, int b, int
         }
   };
   load_block();
-  if (step_factor8<false>(l)) {
+  if (step_factor8<false>(l, col + kStep, lane)) {
     load_block();
-    const unsigned bad = step_factor8<true>(l);
+    const unsigned bad = step_factor8<true>(l, col + kStep, lane);
     if (bad && info && lane == 0) atomicCAS(info, 0, gcol + 8 * b + __ffs(bad));
   }
   step_load8(y, col + hi + lane);  // not kept across the pivots: registers are short
@@ -274,6 +279,13 @@ __device__ __forceinline__ void step_pivots8(double* D, double* pinv, int b, int
     }
     step_store8(col + 32 + lane, y);
   }
+}
+
+// One warp: L_jj, the rounded root of pivot j, which waits in the padding of column j.
+// The substitutions use 1 / L_jj, so the root is off the pivots' chain (pivot times
+// reciprocal, without this, is up to one unit in the last place further off).
+__device__ __forceinline__ void step_roots(double* D, int lane) {
+  for (int j = lane; j < kStep; j += 32) D[j * kStepLd + j] = sqrt(D[j * kStepLd + kStep]);
 }
 
 // The rank-8 update of the diagonal block's columns from 8 (b + 1) on with the
@@ -474,6 +486,7 @@ __device__ __forceinline__ void panel_step_body(double* __restrict__ sm, double*
   double cv[4][4];
   if (warp < ntiles) step_load_c(tile_ptr(warp), ts, cv);
   if (rows_warp) step_rows<2>(A + rc * kStepBlock, D, pinv, 3, 32 * half, lane);
+  if (diag_warp == 0) step_roots(D, lane);
   if (diag_warp == 1) z_substep(3);
   __syncthreads();
 
