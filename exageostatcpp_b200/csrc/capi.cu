@@ -34,8 +34,10 @@ void set_last_error(const char* what, const char* where) {
 // most kPoolKeepBytes of freed memory: the one-shot calls (kriging, MLOE/MMOM,
 // Fisher information) create and destroy their problem every time, and mapping and
 // unmapping its memory cost about 14 us per MB (kriging at N = 10,000: 7 of
-// 25 ms).  What is above goes back at the next synchronisation, and all of it
-// when an allocation of this library fails.
+// 25 ms).  What is above goes back at the next synchronisation.  What is held
+// refuses no other allocation: where one outside the pool (cudaMalloc, another pool,
+// mapped virtual memory) does not fit, the driver takes freed pool memory back by
+// itself, and an allocation of the pool that fails trims it and tries again.
 constexpr unsigned long long kPoolKeepBytes = 1ull << 30;
 
 static cudaMemPool_t device_pool() {
