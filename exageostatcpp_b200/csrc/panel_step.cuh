@@ -9,8 +9,9 @@
 // rows its update needs, so no CTA waits for another one.  It is bound by the
 // chain of 64 dependent pivots, not by work: three dependent launches for the
 // three parts took 58-70 us per step whatever the panel's height, a step now
-// takes about 13 us (N = 1,600, tile 320: panels 1.46 -> 0.44 ms per evaluation, the
-// forward solve below 0.51 -> 0; N = 10,000, tile 960: 11.5 -> 5.0 and 6.9 -> 0).
+// takes 13 to 17 us while every chunk has an SM, 17 to 30 above (N = 1,600, tile 320:
+// panels 1.46 -> 0.44 ms per evaluation, the forward solve below 0.51 -> 0; N = 10,000,
+// tile 960: 11.5 -> 5.0 and 6.9 -> 0).
 // The redundant arithmetic runs on SMs that would otherwise be idle.
 // Outer blocks are two 64-column blocks wide: wider ones make every CTA solve
 // more foreign chunks (each costs as much FP64 time as its own), narrower ones

@@ -23,9 +23,12 @@ namespace egs {
 // One 64-column step of a panel (panel_step_body), and the flush of the step
 // before it: blocks [0, steps) are the step's row chunks, the others copy the
 // scratch slot of the previous step to its place.  CTAS per SM: one leaves the
-// pivot warp enough registers (two cap them at 128 and spill: N = 1,600, 25 chunks,
-// 570 -> 550 us per evaluation with one); two are faster once the chunks fill the
-// SMs more than once (N = 40,000, up to 624: 665 -> 663 ms with two).
+// pivot warp enough registers (two cap them at 128 and spill), two take up to 296
+// chunks in one wave.  The line is where one CTA per SM needs a second wave, more
+// chunks than SMs: first and second step of an outer block at 140 to 148 chunks, 17.3
+// and 13.3 us with one per SM, 19.2 and 13.8 with two; at 150 to 174, 30.3 and 21.8
+// against 29.6 and 17.0 (launch times; panels of N = 16,000, tile 320, up to 246
+// chunks: 6.52 -> 6.19 ms, of N = 40,000, up to 624: 47.0 -> 44.3 ms).
 template <int CTAS>
 __global__ void __launch_bounds__(kStepThreads, CTAS)
 panel_step_kernel(double* col, int ts, int nchunk, int kb, int nb, int gcol, int* info, double* z,
