@@ -1957,8 +1957,9 @@ int egs_mloe_mmom_host(int n_obs, int n_miss, int dts, const double* x_obs, cons
   if ((rc = sync_flags(pt, false)) != EGS_OK || (rc = sync_flags(pa, false)) != EGS_OK) return rc;
   cudaStream_t st = pa->stream, st2 = pt->stream;
   const int ts = pa->ts, nt = pa->nt, np = factor_rows(n_obs), nb = np / kInnerBlock;
-  // targets in groups of at most 512, as the rows of a matrix (64-row chunks)
-  const int group = std::min((n_miss + kInnerBlock - 1) / kInnerBlock * kInnerBlock, 512);
+  // targets in groups of at most 512, as the rows of a matrix (64-row chunks); smaller
+  // groups where the six blocks of a group do not fit beside the factors
+  int group = std::min((n_miss + kInnerBlock - 1) / kInnerBlock * kInnerBlock, 512);
   double *ya = nullptr, *xa = nullptr, *yt = nullptr, *xt = nullptr, *dxm = nullptr, *dym = nullptr, *dots = nullptr;
   long long dummy = 0;
   cudaEvent_t ready = nullptr;
@@ -1968,13 +1969,26 @@ int egs_mloe_mmom_host(int n_obs, int n_miss, int dts, const double* x_obs, cons
     cudaStreamSynchronize(st);
     if (ready) cudaEventDestroy(ready);
   };
-  const size_t block = (size_t)group * np;
-  if ((rc = dev_alloc(&ya, 2 * block, &dummy, st)) || (rc = dev_alloc(&xa, 2 * block, &dummy, st)) ||
-      (rc = dev_alloc(&yt, block, &dummy, st)) || (rc = dev_alloc(&xt, block, &dummy, st)) ||
-      (rc = dev_alloc(&dxm, n_miss, &dummy, st)) || (rc = dev_alloc(&dym, n_miss, &dummy, st)) ||
+  if ((rc = dev_alloc(&dxm, n_miss, &dummy, st)) || (rc = dev_alloc(&dym, n_miss, &dummy, st)) ||
       (rc = dev_alloc(&dots, (size_t)4 * n_miss, &dummy, st))) {
     cleanup();
     return rc;
+  }
+  size_t block = 0;
+  for (;; group = std::max(group / 2 / kInnerBlock, 1) * kInnerBlock) {
+    block = (size_t)group * np;
+    if (!(rc = dev_alloc(&ya, 2 * block, &dummy, st)) && !(rc = dev_alloc(&xa, 2 * block, &dummy, st)) &&
+        !(rc = dev_alloc(&yt, block, &dummy, st)) && !(rc = dev_alloc(&xt, block, &dummy, st)))
+      break;
+    if (rc != EGS_ERR_OOM || group == kInnerBlock) {
+      cleanup();
+      return rc;
+    }
+    for (double** b : {&ya, &xa, &yt, &xt}) {
+      dev_free(*b, st);
+      *b = nullptr;
+    }
+    cudaStreamSynchronize(st);
   }
   if (cudaEventCreateWithFlags(&ready, cudaEventDisableTiming) != cudaSuccess) {
     cudaGetLastError();
