@@ -304,7 +304,7 @@ class Problem:
         _check(self._lib.egs_problem_set_band_method(self._h, int(method)), "set_band_method")
 
     def set_lookahead(self, sms: int) -> None:
-        """SMs given to the look-ahead panel of a mixed problem (0: none); results do not change."""
+        """SMs a mixed problem's off-band update leaves to the next panel (0: no look-ahead); results do not change."""
         _check(self._lib.egs_problem_set_lookahead(self._h, int(sms)), "set_lookahead")
 
     def predict(self, theta, x_miss, y_miss) -> np.ndarray:

@@ -126,7 +126,7 @@ struct egs_batch {
   long long *d_tile_base = nullptr, *d_loc_base = nullptr, *d_partial_base = nullptr;
   int4* d_tinfo = nullptr;
   MaternParams *d_params = nullptr, *h_params = nullptr;
-  double* d_ktab = nullptr;  // B Chebyshev tables of K_nu
+  double* d_ktab = nullptr;  // B polynomial tables of K_nu
   double* h_result = nullptr;
   int *h_info = nullptr, *h_err = nullptr;
   GemmDesc* d_jobs = nullptr;

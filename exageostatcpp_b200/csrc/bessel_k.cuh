@@ -127,7 +127,7 @@ struct MaternParams {
   double mu;         // nu - n
   int n;             // floor(nu + 1/2)
   int kind;          // 0: nu == 1/2, 1: half-integer, 2: general
-  int table;         // 1: general nu <= kKtabMaxNu, evaluated through the Chebyshev table below
+  int table;         // 1: general nu <= kKtabMaxNu, evaluated through the polynomial table below
   int pad_;
 };
 

@@ -97,7 +97,7 @@ struct egs_problem {
   double* result = nullptr;
   int* flags = nullptr;  // [0] potrf info, [1] device wait error
   MaternParams* dparams = nullptr;
-  double* ktab = nullptr;  // Chebyshev table of K_nu for the current theta (kKtabDoubles)
+  double* ktab = nullptr;  // polynomial table of K_nu for the current theta (kKtabDoubles)
   double* pscratch = nullptr;  // solved rows of two panel steps (panel_scratch_doubles)
   // pinned host mirrors
   MaternParams* hparams = nullptr;
@@ -179,8 +179,8 @@ struct egs_problem {
   int4* oz_trsm_targets = nullptr;
   std::vector<OzLaunch> oz_trsm_launch;
   double* W2 = nullptr;  // short panel: diagonal tile, band tiles, identity
-  // look-ahead: the short panel of step k+1 runs on `side` while the off-band
-  // update of step k runs on the other SMs of the problem stream
+  // look-ahead: the short panel of step k+1 is issued on `side` beside the off-band
+  // update of step k, which leaves it lookahead_sms SMs
   cudaStream_t side = nullptr;
   cudaEvent_t ev_band = nullptr, ev_panel = nullptr;
   int lookahead_sms = 0;  // SMs left to the look-ahead panel (0: no look-ahead)
@@ -673,7 +673,8 @@ static int enqueue_short_panel(egs_problem* p, int k, cudaStream_t s) {
 // split the panel rows to FP16, update the FP64 band (Ozaki) and, on all but
 // lookahead_sms SMs, the off-band targets (split-FP16).  The short FP64 panel
 // of step k+1 (diagonal tile, band rows, L^-T) needs only the band update of
-// step k, so it runs on the side stream during the off-band update of step k.
+// step k, so with look-ahead it is issued on the side stream beside the off-band
+// update of step k.
 int enqueue_eval_mixed_ozaki(egs_problem* p) {
   cudaStream_t st = p->stream, side = p->side;
   const int ts = p->ts, nt = p->nt, b = p->mband;

@@ -1,4 +1,4 @@
-// FP64 tensor-core (mma.sync m16n8k16 .f64) and shared/global memory helpers of
+// FP64 tensor-core (mma.sync m16n8k16 .f64) and global memory helpers of
 // the DMMA kernels.  Fragment layout of one warp (g = lane / 4, t = lane % 4):
 //   A: a[2j], a[2j+1] = rows g, g + 8 at k = t + 4j      (j = 0..3)
 //   B: b[i]           = column g at k = t + 4i           (i = 0..3)
@@ -8,14 +8,6 @@
 
 namespace egs {
 
-__device__ __forceinline__ double lds_f64(uint32_t addr) {
-  double v;
-  asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(addr));
-  return v;
-}
-__device__ __forceinline__ void lds_v2f64(uint32_t addr, double& a, double& b) {
-  asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(a), "=d"(b) : "r"(addr));
-}
 __device__ __forceinline__ void ldg_v2f64(const double* p, double& a, double& b) {
   asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(a), "=d"(b) : "l"(p));
 }

@@ -197,6 +197,8 @@ extern "C" int egs_fisher_host(int n, int dts, const double* x, const double* y,
   int ts = 0, nt = 0;
   cudaStream_t st = nullptr;
   problem_tiles(p, &tiles, &dx, &dy, &ts, &nt, &st);
+  // The sweeps below have no such limit: it is the entry's, kept from the form that
+  // factored a matrix of 2 nt tile rows, so that what it refuses does not change.
   if (lower_tiles(2 * nt) > 65535) {
     set_last_error("more than 180 tile rows; use a larger dts", "egs_fisher_host");
     return EGS_ERR_INVALID;

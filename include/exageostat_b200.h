@@ -103,11 +103,13 @@ EGS_API int egs_problem_set_precision(egs_problem* p, int precision, int band_ti
 EGS_API int egs_problem_set_band_method(egs_problem* p, int method);
 
 /* Look-ahead of a mixed problem (Ozaki band method): the FP64 panel of step
- * k+1 (diagonal tile, band rows, L^-1) runs on `sms` SMs beside the off-band
- * update of step k, which keeps the other SMs; 0 runs them one after the
- * other (the default: at N = 102,400 the off-band update loses as much time
- * to the reserved SMs as the overlap hides).  A scheduling choice only:
- * results are bit-identical either way. */
+ * k+1 (diagonal tile, band rows, L^-1) is issued beside the off-band update of
+ * step k, which leaves `sms` SMs to it; the panel's own launches are not
+ * limited to them.  0, the default, runs the two one after the other.  At
+ * N = 102,400 the update loses at least as much time to the SMs it leaves as the
+ * overlap hides (0 / 8 / 16 / 32 SMs: 1,419 / 1,420 / 1,435 / 1,490 ms an evaluation); at
+ * N = 20,011 it gains up to 3 % (0 / 8 / 16 / 32 / 48: 30.7 / 30.4 / 30.2 / 29.9 / 29.8 ms).
+ * A scheduling choice only: results are bit-identical either way. */
 EGS_API int egs_problem_set_lookahead(egs_problem* p, int sms);
 
 /* Create a problem directly in the given precision (EGS_PRECISION_DOUBLE or
@@ -422,10 +424,11 @@ EGS_API int egs_mloe_mmom_host(int n_obs, int n_miss, int dts, const double* x_o
  * column-major (3 x 3).  Replaces LinearAlgebraMethods<T>::ExaGeoStatFisherTile
  * (src/linear-algebra-solvers/LinearAlgebraMethods.cpp:1133-1306) with the
  * derivative kernels UnivariateMaternDdsigmaSquare / Dbeta / Dnu
- * (src/kernels/concrete/); d K_nu / d nu by Richardson-extrapolated central
- * differences (steps 1e-3, 5e-4) where the reference takes a forward one
- * (step 1e-9, BasselFunction.cpp:23-33).
- * Works in dense n x n buffers (about 8 n^2 doubles). */
+ * (src/kernels/concrete/); the derivative in nu is a six-point central difference of
+ * x^nu K_nu (step 2e-3) where the reference takes a forward one of K_nu (step
+ * 1e-9, BasselFunction.cpp:23-33).
+ * Holds about 6.5 n^2 doubles on the device.  Refused (EGS_ERR_INVALID) beyond
+ * 180 tile rows. */
 EGS_API int egs_fisher_host(int n, int dts, const double* x, const double* y, const double* theta,
                             double* fisher_inverse);
 

@@ -33,8 +33,8 @@ def test_entries_equal_those_of_the_division(beta):
     dx, dy = torch.tensor(x, device="cuda"), torch.tensor(y, device="cuda")
     a = torch.zeros(n * n, dtype=torch.float64, device="cuda")
     ptr = [ctypes.c_void_p(t.data_ptr()) for t in (a, dx, dy)]
-    egs._check(lib.egs_matern_block(ptr[0], n, n, n, ptr[1], ptr[2], ptr[1], ptr[2], theta.ctypes.data_as(egs._D), 0, None),
-               "egs_matern_block")
+    egs._check(lib.egs_matern_block(ptr[0], n, n, n, ptr[1], ptr[2], ptr[1], ptr[2], theta.ctypes.data_as(egs._D), 0,
+                                    None), "egs_matern_block")
     torch.cuda.synchronize()
     ref = np.tril(a.cpu().numpy().reshape(n, n).T)
     assert np.all(np.isfinite(ref))
